@@ -51,11 +51,11 @@ class Params(C.Structure):
 
 
 def build(reference: Optional[str] = None, quiet: bool = True) -> None:
-    """Compile the restatement, and the reference library when the reference tree exists."""
+    """Compile the restatement, and the reference library when the reference's sources exist."""
     out = subprocess.DEVNULL if quiet else None
     subprocess.run(["make", "-C", HERE, "all"], check=True, stdout=out)
     ref = reference or REFERENCE_DIR
-    if os.path.isdir(ref):
+    if os.path.isfile(os.path.join(ref, "Solver.cpp")):
         subprocess.run(["make", "-C", HERE, "ref", f"REFERENCE={ref}"], check=True, stdout=out)
 
 
