@@ -82,7 +82,7 @@ constexpr int STATS_SLOTS = 16;
 // launch with programmatic stream serialization (the kernel starts with pdl_prologue), so the
 // launch of a kernel overlaps the tail of the one before it in the stream or graph
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A &&... args)
+inline cudaError_t launch_pdl_smem(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&... args)
 {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -90,11 +90,16 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaS
     cudaLaunchConfig_t c{};
     c.gridDim = grid;
     c.blockDim = block;
-    c.dynamicSmemBytes = 0;
+    c.dynamicSmemBytes = smem;
     c.stream = s;
     c.attrs = at;
     c.numAttrs = 1;
     return cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A &&... args)
+{
+    return launch_pdl_smem(kernel, grid, block, 0, s, std::forward<A>(args)...);
 }
 
 // keeps the first failure of a sequence of launches (err may be null)

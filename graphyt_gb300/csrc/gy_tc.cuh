@@ -85,7 +85,8 @@ __device__ __forceinline__ void mbar_init(uint64_t *mbar, uint32_t count)
 
 // Wait for the phase with the given parity to complete; false if the wait gave up.  The
 // poll is the non-blocking test_wait with a short sleep between polls, so the bound on the
-// wait is the poll count times the sleep (a fraction of a second).
+// wait is the poll count times the sleep (a fraction of a second); the first polls, which cover
+// an MMA of a few hundred cycles, do not sleep.
 __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity)
 {
     const uint32_t a = smem_u32(mbar);
@@ -99,7 +100,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity)
             : "r"(a), "r"(parity)
             : "memory");
         if (done) return true;
-        __nanosleep(32);
+        if (it >= 64) __nanosleep(32);
     }
     return false;
 }

@@ -240,3 +240,63 @@ def test_mlp_training_fits_a_smooth_map(gpu_lib, torch_cuda):
     want = f(xv.astype(np.float64))
     err = np.linalg.norm(Y.cpu().numpy() - want) / np.linalg.norm(want)
     assert err <= 0.15, err
+
+
+@pytest.mark.parametrize("n,offset,scale", [(129, 1, 1.0), (120_001, 3, 1.0), (120_001, 4, 1.0), (1000, 0, 300.0)])
+def test_mlp_forward_tiles_alignment_and_saturation(gpu_lib, torch_cuda, n, offset, scale):
+    """Rows that do not start on 16 bytes take the 4-byte loads, more rows than one wave of tiles
+    loop: row for row the bits of a call on an aligned copy of 128 rows (a row's arithmetic does
+    not depend on its tile).  Inputs hundreds of deviations out drive the hidden activations past
+    exp's overflow: the outputs stay within the forward test's 2e-3 of the reference."""
+    torch = torch_cuda
+    from graphyt_gb300 import _lib
+    rng = np.random.default_rng(n + offset)
+    prm, _ = mlp_params(rng, rng.standard_normal(16), 0.5 + rng.random(16), rng.standard_normal(7), 0.5 + rng.random(7))
+    x = (scale * rng.standard_normal((n, 16))).astype(np.float32)
+    P = torch.from_numpy(prm).cuda()
+    flat = torch.zeros(n * 16 + offset, dtype=torch.float32, device="cuda")
+    flat[offset:] = torch.from_numpy(x).cuda().reshape(-1)
+
+    def forward(ptr, rows):
+        Y = torch.full((rows, 7), float("nan"), dtype=torch.float32, device="cuda")
+        st = torch.zeros(1, dtype=torch.int32, device="cuda")
+        assert gpu_lib.gy_mlp_forward(_ptr(P), ctypes.c_void_p(ptr), rows, _ptr(Y), _ptr(st),
+                                      ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == _lib.GY_OK
+        torch.cuda.synchronize()
+        assert int(st.item()) == 0
+        return Y.cpu().numpy()
+
+    got = forward(flat.data_ptr() + 4 * offset, n)
+    for first in (0, (n // 2) & ~127, n - 128):
+        X = torch.from_numpy(np.ascontiguousarray(x[first:first + 128])).cuda()
+        assert np.array_equal(forward(X.data_ptr(), 128), got[first:first + 128])
+    with np.errstate(over="ignore"):
+        want = mlp_reference(x.astype(np.float64), prm, True)
+    assert np.linalg.norm(got - want) <= 2e-3 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("steps", [1, 2, 15, 16, 17, 33])
+def test_mlp_training_takes_every_step(gpu_lib, torch_cuda, steps):
+    """Steps are replayed sixteen to a graph with the remainder in another: the loss a call of
+    k + 1 steps reports, that of its last step, is the loss of the parameters k steps leave (data
+    of one row, so that every batch is the same; 1e-4 for the order of the FP32 atomics)."""
+    torch = torch_cuda
+    from graphyt_gb300 import _lib
+    rng = np.random.default_rng(9)
+    prm, _ = mlp_params(rng, np.zeros(16), np.ones(16), np.zeros(7), np.ones(7))
+    X = torch.from_numpy(np.tile(rng.standard_normal((1, 16)).astype(np.float32), (128, 1))).cuda()
+    T = torch.from_numpy(np.tile(rng.standard_normal((1, 7)).astype(np.float32), (128, 1))).cuda()
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def train(k):
+        P, loss = torch.from_numpy(prm).cuda(), ctypes.c_float()
+        assert gpu_lib.gy_mlp_train(_ptr(P), _ptr(X), _ptr(T), 128, k, 128, 1e-3, 7, 0, ctypes.byref(loss), None,
+                                    stream) == _lib.GY_OK
+        return P, loss.value
+
+    P, _ = train(steps)
+    G, Lo = torch.zeros(len(prm), device="cuda"), torch.zeros(1, device="cuda")
+    assert gpu_lib.gy_mlp_grad(_ptr(P), _ptr(X), _ptr(T), 128, _ptr(G), _ptr(Lo), None, stream) == _lib.GY_OK
+    torch.cuda.synchronize()
+    _, loss = train(steps + 1)
+    assert abs(loss - float(Lo.item())) <= 1e-4 * abs(loss)
