@@ -132,6 +132,7 @@ struct gy_solver {
     // stepping
     double t_prev = 0.0;
     long long steps = 0;
+    int epoch = 0;                          // the running step's mark of an active node block
     long long since_sort = 1 << 30;
     bool tables_valid = false;
     bool phase_timing = false;
@@ -913,6 +914,7 @@ static StepScalars make_scalars(const gy_solver *h, int step)
     sc.multi_body = h->multi ? 1 : 0;
     sc.init_volume = (float)(h->g.is3d ? h->psep * h->psep * h->psep : h->psep * h->psep);
     sc.step = step;
+    sc.epoch = h->epoch;
     return sc;
 }
 
@@ -1003,10 +1005,10 @@ static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
     if (tev) cudaEventRecord(tev[2], s);
     // (c) periodic fold, nodal solve, grid BCs
     launch_fold(h->nb, a, s);
-    launch_solve(h->nb, a, h->opt.keep_node_fields != 0, s);
+    launch_solve(h->nb, a, h->opt.keep_node_fields != 0, h->thermal, s);
     if (tev) cudaEventRecord(tev[3], s);
     // (d) G2P + particle BCs + update + constitutive + damage, written in sorted order, with
-    // the conservation sums of the updated state (their partials zeroed by the compaction)
+    // the conservation sums of the updated state (their partials zeroed by the fold)
     if (h->surr_on) cudaMemsetAsync(h->d_pend_n, 0, sizeof(unsigned int), s);
     launch_g2p_update(src, dst, perm, skey, h->n, h->d_seg, nseg, h->g2p_grid, h->nb, a,
                       h->opt.track_normals != 0, h->opt.check_finite != 0, h->has_dp, s,
@@ -1051,6 +1053,7 @@ static gy_status enqueue_step(gy_solver *h, double t, int step)
     {
         const int slot = (int)(h->ring_pos++ % gy_solver::kRing);
         if (h->ring_busy[slot]) CK(h, cudaEventSynchronize(h->ring_ev[slot]));
+        h->epoch = h->epoch == 0x7fffffff ? 1 : h->epoch + 1;
         h->h_ring[slot] = make_scalars(h, step);
         CK(h, cudaMemcpyAsync(h->d_sc, &h->h_ring[slot], sizeof(StepScalars), cudaMemcpyHostToDevice, s));
         CK(h, cudaEventRecord(h->ring_ev[slot], s));

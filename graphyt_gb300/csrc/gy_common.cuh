@@ -97,6 +97,7 @@ struct StepScalars {
     int multi_body;
     float init_volume;        // psep^3 (psep^2 in 2D): volume before the first update
     int step;                 // the step index (sampling of logged Drucker-Prager returns)
+    int epoch;                // positive, different in every step of a handle (active node blocks)
 };
 
 // ---------------------------------------------------------------------------------------

@@ -52,11 +52,11 @@ __device__ __forceinline__ void cp_async4(void *smem, const void *gmem)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// Mark the node's 4x4x4 block active: a plain store (no round trip); k_compact_active turns
-// the flags into the solve's list.
-__device__ __forceinline__ void mark_node(const NodeBufs &nb, int i, int j, int k, const GridGeom &g)
+// Mark the node's 4x4x4 block active in this step: a plain store (no round trip) of the step's
+// epoch, which no earlier step has written, so that nothing clears the flags.
+__device__ __forceinline__ void mark_node(const NodeBufs &nb, int i, int j, int k, const GridGeom &g, int epoch)
 {
-    nb.flags[node_block(i, j, k, g)] = 1;
+    nb.flags[node_block(i, j, k, g)] = epoch;
 }
 
 struct PState {
@@ -264,8 +264,9 @@ template <bool THERMAL>
 __global__ void __launch_bounds__(PC_THREADS, GY_PC_MINB) k_p2g_cols(PView P, const int *perm, const int *skey, long long n,
                                                          const int *seg_start, const int *nseg_ptr, int sorted,
                                                          NodeBufs nb, GridGeom g, const float4 *therm, float2 *tnode,
-                                                         const DevMaterial *mats)
+                                                         const DevMaterial *mats, const StepScalars *sc)
 {
+    const int epoch = sc->epoch;
     constexpr int NF = P2G_FIELDS + (THERMAL ? 2 : 0);
     __shared__ float tile[NF * PT_NODES];
     __shared__ float4 QTs[THERMAL ? 2 * PC_NP : 1];
@@ -479,7 +480,7 @@ __global__ void __launch_bounds__(PC_THREADS, GY_PC_MINB) k_p2g_cols(PView P, co
                 atomicAdd(&tnode[nd].x, tile[7 * PT_NODES + t]);
                 atomicAdd(&tnode[nd].y, tile[8 * PT_NODES + t]);
             }
-            mark_node(nb, ni, nj, nk, g);
+            mark_node(nb, ni, nj, nk, g, epoch);
         }
         __syncthreads();
     }
@@ -543,6 +544,7 @@ __global__ void __launch_bounds__(PP_THREADS, THERMAL ? GY_PP_MINB_TH : GY_PP_MI
     __shared__ int wcount[PP_THREADS / 32];
     __shared__ long long s_end;
     const GridGeom &g = a.g;
+    const int epoch = a.sc->epoch;
     const int nseg = *nseg_ptr;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;
@@ -781,7 +783,7 @@ __global__ void __launch_bounds__(PP_THREADS, THERMAL ? GY_PP_MINB_TH : GY_PP_MI
                 atomicAdd(&tnode[nd].x, tile[7 * PT_NODES + t]);
                 atomicAdd(&tnode[nd].y, tile[8 * PT_NODES + t]);
             }
-            mark_node(nb, ni, nj, nk, g);
+            mark_node(nb, ni, nj, nk, g, epoch);
         }
         __syncthreads();
     }
@@ -816,6 +818,7 @@ __global__ void __launch_bounds__(P2G_CH) k_p2g_multi_tiled(PView P, const int *
     const bool scatter_lane = lane < 27;
     const float grx = a.sc->gravity[0], gry = a.sc->gravity[1], grz = a.sc->gravity[2];
     const float init_vol = a.sc->init_volume;
+    const int epoch = a.sc->epoch;
     for (int sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
         const long long start = seg_start[sgi];
         const int blk = seg_block(skey, start);
@@ -1047,7 +1050,7 @@ __global__ void __launch_bounds__(P2G_CH) k_p2g_multi_tiled(PView P, const int *
                     red_add4(&nb.bacc1[0][nd], f[4 * PT_NODES], f[5 * PT_NODES], f[6 * PT_NODES], 0.f);
                     red_add4(&nb.bnrm[0][nd], f[14 * PT_NODES], f[15 * PT_NODES], f[16 * PT_NODES], 0.f);
                 }
-                mark_node(nb, ni, nj, nk, g);
+                mark_node(nb, ni, nj, nk, g, epoch);
                 continue;
             }
 #pragma unroll
@@ -1058,7 +1061,7 @@ __global__ void __launch_bounds__(P2G_CH) k_p2g_multi_tiled(PView P, const int *
                 red_add4(&nb.bacc1[sl][nd], b[4 * PT_NODES], b[5 * PT_NODES], b[6 * PT_NODES], 0.f);
                 red_add4(&nb.bnrm[sl][nd], b[7 * PT_NODES], b[8 * PT_NODES], b[9 * PT_NODES], 0.f);
             }
-            mark_node(nb, ni, nj, nk, g);
+            mark_node(nb, ni, nj, nk, g, epoch);
         }
     }
 }
@@ -1111,7 +1114,7 @@ void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, c
                 tgrid = sms * std::max(b, 1);
             }
             k_p2g_cols<true><<<tgrid, PC_THREADS, 0, s>>>(p, perm, skey, n, seg_start, nseg, perm ? 1 : 0, nb, a.g,
-                                                           therm, tnode, a.mats);
+                                                           therm, tnode, a.mats, a.sc);
         } else if (lanes == 3) {
             static int pgrid = 0;  // persistent grid of the plane-lane kernel (its own occupancy)
             if (pgrid == 0) {
@@ -1125,7 +1128,7 @@ void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, c
                                                               nullptr, nullptr);
         } else {
             k_p2g_cols<false><<<persist_grid, PC_THREADS, 0, s>>>(p, perm, skey, n, seg_start, nseg, perm ? 1 : 0, nb,
-                                                                   a.g, nullptr, nullptr, nullptr);
+                                                                   a.g, nullptr, nullptr, nullptr, a.sc);
         }
     }
     note_launch(1);
@@ -1142,61 +1145,96 @@ int p2g_blocks_per_sm()
 // periodic fold, Grid.cpp:310-795: node i and node N-3+i (i < 3) both take their sum, for
 // mass, momentum and force of the centre-of-mass field and both body fields.
 
-__device__ __forceinline__ bool fold4(float4 *arr, long long p, long long q)
-{
-    const float4 x = arr[p], y = arr[q];
-    const float4 s = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
-    arr[p] = s;
-    arr[q] = s;
-    return s.x != 0.f || s.y != 0.f || s.z != 0.f || s.w != 0.f;
-}
-
+// The reference folds axis after axis; a node near an edge or corner is thus summed over 4 or 8
+// images, all of which end with that sum.  A thread takes all images of one node, summed in the
+// order of the three passes, so that one launch does what three dependent ones did (three
+// launches of 3-5 us each on grids where nearly every pair is empty).  It also zeroes the
+// conservation partials the step's G2P adds into (stats, may be null).
 template <bool MULTI>
-__global__ void k_fold(NodeBufs nb, GridGeom g, int axis)
+__global__ void __launch_bounds__(256) k_fold(NodeBufs nb, GridGeom g, const StepScalars *sc, double *stats)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int d0, d1;
-    if (axis == 0) { d0 = g.ny; d1 = g.nz; }
-    else if (axis == 1) { d0 = g.nx; d1 = g.nz; }
-    else { d0 = g.nx; d1 = g.ny; }
-    const long long plane = (long long)d0 * d1;
-    if (t >= 3 * plane) return;
-    const int l = (int)(t / plane);
-    const long long r = t - (long long)l * plane;
-    const int a0 = (int)(r % d0), a1 = (int)(r / d0);
-    int pi, pj, pk, qi, qj, qk;
-    if (axis == 0) { pi = l; pj = a0; pk = a1; qi = g.nx - 3 + l; qj = a0; qk = a1; }
-    else if (axis == 1) { pi = a0; pj = l; pk = a1; qi = a0; qj = g.ny - 3 + l; qk = a1; }
-    else { pi = a0; pj = a1; pk = l; qi = a0; qj = a1; qk = g.nz - 3 + l; }
-    // the accumulators of a node block P2G (or an earlier axis' fold) did not flag are all
-    // zero: a pair of such nodes folds to zeros already in place
-    if (!nb.flags[node_block(pi, pj, pk, g)] && !nb.flags[node_block(qi, qj, qk, g)]) return;
-    const long long p = node_index(pi, pj, pk, g), q = node_index(qi, qj, qk, g);
-    bool any = fold4(nb.acc0, p, q);
-    any |= fold4(nb.acc1, p, q);
-    if (MULTI) {
-        for (int b = 0; b < 2; b++) {
-            any |= fold4(nb.bacc0[b], p, q);
-            any |= fold4(nb.bacc1[b], p, q);
+    pdl_prologue();
+    if (stats && blockIdx.x == 0)
+        for (int q = threadIdx.x; q < STATS_SLOTS * 8; q += blockDim.x) stats[q] = 0.0;
+    // the representative of an orbit has every coordinate below N - 3 and one of them below 3:
+    // the slab i < 3, then j < 3 of the rest, then k < 3 of the rest (3D only)
+    const int mx = g.nx - 3, my = g.ny - 3, mz = g.is3d ? g.nz - 3 : 1;
+    const int c0 = 3 * my * mz, c1 = (mx - 3) * 3 * mz, c2 = g.is3d ? (mx - 3) * (my - 3) * 3 : 0;
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    int i, j, k;
+    if (t < c0) {
+        i = t % 3; t /= 3;
+        j = t % my; k = t / my;
+    } else if ((t -= c0) < c1) {
+        i = 3 + t % (mx - 3); t /= mx - 3;
+        j = t % 3; k = t / 3;
+    } else if ((t -= c1) < c2) {
+        i = 3 + t % (mx - 3); t /= mx - 3;
+        j = 3 + t % (my - 3); k = t / (my - 3);
+    } else {
+        return;
+    }
+    const bool fx = i < 3, fy = j < 3, fz = g.is3d && k < 3;
+    const int epoch = sc->epoch;
+    // image e: bit 0 the x partner, bit 1 the y partner, bit 2 the z partner
+    unsigned img = 1u;
+    if (fx) img |= img << 1;
+    if (fy) img |= img << 2;
+    if (fz) img |= img << 4;
+    int nd[8];
+    bool live = false;
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+        const int ei = (e & 1) ? mx + i : i, ej = (e & 2) ? my + j : j, ek = (e & 4) ? mz + k : k;
+        const bool on = (img >> e) & 1u;
+        nd[e] = on ? node_index(ei, ej, ek, g) : 0;
+        // the accumulators of a node block P2G did not flag are all zero
+        if (on) live = live || nb.flags[node_block(ei, ej, ek, g)] == epoch;
+    }
+    if (!live) return;
+    bool any = false;
+    const int na = MULTI ? 6 : 2;
+    for (int f = 0; f < na; f++) {
+        float4 *arr = f == 0 ? nb.acc0 : f == 1 ? nb.acc1 : (f & 1) ? nb.bacc1[(f - 2) >> 1] : nb.bacc0[(f - 2) >> 1];
+        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 v[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[e] = ((img >> e) & 1u) ? arr[nd[e]] : z4;
+        // the pairs of each axis in turn, as the three passes add them
+#pragma unroll
+        for (int w = 1; w < 8; w <<= 1) {
+            if (!((w == 1 && fx) || (w == 2 && fy) || (w == 4 && fz))) continue;
+#pragma unroll
+            for (int e = 0; e < 8; e++)
+                if (!(e & w)) {
+                    v[e].x += v[e | w].x;
+                    v[e].y += v[e | w].y;
+                    v[e].z += v[e | w].z;
+                    v[e].w += v[e | w].w;
+                }
         }
+        const float4 s = v[0];
+        any = any || s.x != 0.f || s.y != 0.f || s.z != 0.f || s.w != 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; e++)
+            if ((img >> e) & 1u) arr[nd[e]] = s;
     }
-    if (any) {
-        mark_node(nb, pi, pj, pk, g);
-        mark_node(nb, qi, qj, qk, g);
-    }
+    if (any)
+#pragma unroll
+        for (int e = 0; e < 8; e++)
+            if ((img >> e) & 1u)
+                mark_node(nb, (e & 1) ? mx + i : i, (e & 2) ? my + j : j, (e & 4) ? mz + k : k, g, epoch);
 }
 
 void launch_fold(const NodeBufs &nb, const StepArgs &a, cudaStream_t s)
 {
     const GridGeom &g = a.g;
-    const int naxes = g.is3d ? 3 : 2;
-    for (int ax = 0; ax < naxes; ax++) {
-        const long long plane = ax == 0 ? (long long)g.ny * g.nz : ax == 1 ? (long long)g.nx * g.nz : (long long)g.nx * g.ny;
-        const unsigned grid = (unsigned)((3 * plane + 255) / 256);
-        if (a.multi_body) k_fold<true><<<grid, 256, 0, s>>>(nb, g, ax);
-        else k_fold<false><<<grid, 256, 0, s>>>(nb, g, ax);
-        note_launch(1);
-    }
+    const long long mx = g.nx - 3, my = g.ny - 3, mz = g.is3d ? g.nz - 3 : 1;
+    const long long orbits = 3 * my * mz + (mx - 3) * 3 * mz + (g.is3d ? (mx - 3) * (my - 3) * 3 : 0);
+    const unsigned grid = (unsigned)((orbits + 255) / 256);
+    if (a.multi_body) launch_pdl(k_fold<true>, grid, 256, s, nb, g, a.sc, a.stats);
+    else launch_pdl(k_fold<false>, grid, 256, s, nb, g, a.sc, a.stats);
+    note_launch(1);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1425,23 +1463,36 @@ __device__ __forceinline__ bool solve_node(const NodeBufs &nb, const StepArgs &a
     return active;
 }
 
+// How many blocks' flags a warp of the solve reads at once: a warp takes every nw-th node block,
+// so that the active ones, which lie together, spread over all warps; with the flags read in the
+// solve itself there is no list to build first (a launch of 3 us).
+constexpr int SOLVE_FLAGS = 4;
+
 // Single-body nodal solve (Grid.cpp:9-245 without contact, then the grid BCs): one warp per
-// listed block, each lane owns nodes lane and lane + 32, and all loads of both nodes are
-// issued before the first result is needed.
-__global__ void __launch_bounds__(256) k_solve_single(NodeBufs nb, StepArgs a, int keep)
+// active block, each lane owns nodes lane and lane + 32, and all loads of both nodes are
+// issued before the first result is needed.  want_list: also list the active blocks (heat
+// conduction clears its node fields over them).
+__global__ void __launch_bounds__(256) k_solve_single(NodeBufs nb, StepArgs a, int keep, int want_list)
 {
+    pdl_prologue();
     const GridGeom &g = a.g;
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nw = (int)((gridDim.x * blockDim.x) >> 5);
-    const int nact = *nb.active_n;
+    const int nnb = (int)g.nnb, epoch = a.sc->epoch;
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     const float dtn = a.sc->dt_node;
     const float grx = a.sc->gravity[0], gry = a.sc->gravity[1], grz = a.sc->gravity[2];
     const int fixed_bcs = a.sc->fixed_grid_bcs;
     int count = 0;
-    for (int w = gw; w < nact; w += nw) {
-        const int blk = nb.active_list[w];
+    for (int w0 = gw; w0 < nnb; w0 += SOLVE_FLAGS * nw) {
+      unsigned active = 0u;
+#pragma unroll
+      for (int u = 0; u < SOLVE_FLAGS; u++)
+          active |= w0 + u * nw < nnb && nb.flags[w0 + u * nw] == epoch ? 1u << u : 0u;
+      for (; active; active &= active - 1u) {
+        const int blk = w0 + (__ffs(active) - 1) * nw;
+        if (want_list && lane == 0) nb.active_list[atomicAdd(nb.active_n, 1)] = blk;
         const int bx = blk % g.nnbx, tb = blk / g.nnbx;
         const int by = tb % g.nnby, bz = tb / g.nnby;
         int nd[2];
@@ -1458,7 +1509,6 @@ __global__ void __launch_bounds__(256) k_solve_single(NodeBufs nb, StepArgs a, i
             A1[h] = in[h] ? nb.acc1[nd[h]] : z4;
             bt[h] = (in[h] && nb.bc_type) ? (int)nb.bc_type[nd[h]] : 0;
         }
-        if (lane == 0) nb.flags[blk] = 0;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             if (!in[h]) continue;
@@ -1497,6 +1547,7 @@ __global__ void __launch_bounds__(256) k_solve_single(NodeBufs nb, StepArgs a, i
                 nb.out_force[nd[h]] = make_float4(F.x, F.y, F.z, 0.f);
             }
         }
+      }
     }
     if (nb.active_count) {
         for (int off = 16; off > 0; off >>= 1) count += __shfl_down_sync(0xffffffffu, count, off);
@@ -1504,43 +1555,31 @@ __global__ void __launch_bounds__(256) k_solve_single(NodeBufs nb, StepArgs a, i
     }
 }
 
-// The flagged node blocks, appended to the solve's list: one ballot and one atomic per warp.
-// It also zeroes the conservation partials the step's G2P adds into (stats, may be null).
-__global__ void k_compact_active(NodeBufs nb, int nnb, double *stats)
-{
-    const int lane = threadIdx.x & 31;
-    if (stats && blockIdx.x == 0)
-        for (int q = threadIdx.x; q < STATS_SLOTS * 8; q += blockDim.x) stats[q] = 0.0;
-    for (int b0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; b0 < nnb; b0 += gridDim.x * blockDim.x) {
-        const int b = b0 + lane;
-        const bool f = b < nnb && nb.flags[b] != 0;
-        const unsigned m = __ballot_sync(0xffffffffu, f);
-        if (!m) continue;
-        int base = 0;
-        if (lane == 0) base = atomicAdd(nb.active_n, __popc(m));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (f) nb.active_list[base + __popc(m & ((1u << lane) - 1u))] = b;
-    }
-}
-
-// Multi-body nodal solve with contact: two warps per active node block from the list P2G
-// and the fold built (32 nodes each); the block's flag is cleared for the next step.
+// Multi-body nodal solve with contact: two warps per active node block (32 nodes each).
 #ifndef GY_SOLVE_MINB
 #define GY_SOLVE_MINB 5  // resident 256-thread CTAs per SM the multi-body solve is register-capped to (48)
 #endif
 template <bool MULTI>
-__global__ void __launch_bounds__(256, GY_SOLVE_MINB) k_solve_list(NodeBufs nb, StepArgs a, int keep)
+__global__ void __launch_bounds__(256, GY_SOLVE_MINB) k_solve_multi(NodeBufs nb, StepArgs a, int keep, int want_list)
 {
+    pdl_prologue();
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nw = (int)((gridDim.x * blockDim.x) >> 5);
-    const int nact = *nb.active_n;
+    const int nnb = (int)a.g.nnb, epoch = a.sc->epoch;
     int count = 0;
     // one warp per half block (32 nodes), so the two halves' loads are in flight together
-    for (int w = gw; w < 2 * nact; w += nw) {
-        const long long blk = nb.active_list[w >> 1];
-        count += solve_node<MULTI>(nb, a, keep, blk, lane + 32 * (w & 1)) ? 1 : 0;
-        if (lane == 0 && (w & 1) == 0) nb.flags[blk] = 0;
+    const int half = gw & 1, step = nw >> 1;  // nw is even
+    for (int w0 = gw >> 1; w0 < nnb; w0 += SOLVE_FLAGS * step) {
+        unsigned active = 0u;
+#pragma unroll
+        for (int u = 0; u < SOLVE_FLAGS; u++)
+            active |= w0 + u * step < nnb && nb.flags[w0 + u * step] == epoch ? 1u << u : 0u;
+        for (; active; active &= active - 1u) {
+            const int blk = w0 + (__ffs(active) - 1) * step;
+            if (want_list && half == 0 && lane == 0) nb.active_list[atomicAdd(nb.active_n, 1)] = blk;
+            count += solve_node<MULTI>(nb, a, keep, blk, lane + 32 * half) ? 1 : 0;
+        }
     }
     if (nb.active_count) {
         for (int off = 16; off > 0; off >>= 1) count += __shfl_down_sync(0xffffffffu, count, off);
@@ -1548,18 +1587,19 @@ __global__ void __launch_bounds__(256, GY_SOLVE_MINB) k_solve_list(NodeBufs nb, 
     }
 }
 
-void launch_solve(const NodeBufs &nb, const StepArgs &a, bool keep_node_fields, cudaStream_t s)
+void launch_solve(const NodeBufs &nb, const StepArgs &a, bool keep_node_fields, bool want_list, cudaStream_t s)
 {
-    int dev = 0, sms = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long cgrid = std::min<long long>((a.g.nnb + 255) / 256, (long long)sms * 8);
-    k_compact_active<<<(unsigned)std::max<long long>(cgrid, 1), 256, 0, s>>>(nb, (int)a.g.nnb, a.stats);
-    note_launch(1);
-    long long grid = std::min<long long>((a.g.nnb + 7) / 8, (long long)sms * 16);  // 8 warps per CTA
-    if (grid < 1) grid = 1;
-    if (a.multi_body) k_solve_list<true><<<(unsigned)grid, 256, 0, s>>>(nb, a, keep_node_fields ? 1 : 0);
-    else k_solve_single<<<(unsigned)grid, 256, 0, s>>>(nb, a, keep_node_fields ? 1 : 0);
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
+    const int keep = keep_node_fields ? 1 : 0, list = want_list ? 1 : 0;
+    const long long warps = a.multi_body ? 2 * a.g.nnb : a.g.nnb;
+    const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>((warps + 7) / 8, (long long)sms * 16));
+    if (a.multi_body) launch_pdl(k_solve_multi<true>, grid, 256, s, nb, a, keep, list);
+    else launch_pdl(k_solve_single, grid, 256, s, nb, a, keep, list);
     note_launch(1);
 }
 

@@ -35,8 +35,8 @@ struct NodeBufs {
     float4 *bgv[2], *bga[2];      // solved per slot: (m, v), (a, -); slot 0's are gv / ga
     float4 *nrm_out[2];           // normalised slot normals (only when normals are tracked)
     int2 *body;                   // body slot objects (dense ids) or -1
-    int *flags;                   // active 4x4x4 node blocks (set by P2G / fold, cleared by the solve)
-    int *active_list;             // node blocks marked this step, in marking order
+    int *flags;                   // per 4x4x4 node block: the epoch of the last step P2G or the fold wrote it in
+    int *active_list;             // node blocks marked this step (when the solve is asked for the list)
     int *active_n;                // length of active_list
     unsigned char *has_rigid;     // bit0: slot 0 rigid, bit1: slot 1 rigid
     int *active_count;            // nodes with mass (stats)
@@ -122,7 +122,8 @@ void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, c
                 int *ndefer = nullptr);
 void launch_fold(const NodeBufs &nb, const StepArgs &a, cudaStream_t s);
 void launch_block_body(const NodeBufs &nb, const GridGeom &g, cudaStream_t s);
-void launch_solve(const NodeBufs &nb, const StepArgs &a, bool keep_node_fields, cudaStream_t s);
+// want_list: fill active_list / active_n (zeroed by the caller's block heads)
+void launch_solve(const NodeBufs &nb, const StepArgs &a, bool keep_node_fields, bool want_list, cudaStream_t s);
 // therm / tnode non-null: the single-body kernel also runs the heat conduction G2P and the
 // temperature update (multi-body problems run launch_thermal_g2p instead)
 void launch_g2p_update(const PView &src, const PView &dst, const int *perm, const int *skey, long long n,
