@@ -21,11 +21,13 @@ using namespace gy;
 struct StepVariant {
     int cur;       // slab read this step
     int sk;        // sorted-key buffer written by this step's sort (the other one is read)
-    int sort;      // 0 none, 1 incremental, 2 full
+    int sort;      // 0 none, 1 incremental, 2 full, 3 block merge
     int tables;    // 0 none, 1 rebuild body tables, 2 rebuild from the initial keys
+    int blocks;    // G2P keeps the block merge sort's counts (else it flags the movers)
+    int fb;        // first-position buffer this step's block scan writes
     bool operator==(const StepVariant &o) const
     {
-        return cur == o.cur && sk == o.sk && sort == o.sort && tables == o.tables;
+        return cur == o.cur && sk == o.sk && sort == o.sort && tables == o.tables && blocks == o.blocks && fb == o.fb;
     }
 };
 
@@ -76,6 +78,7 @@ struct gy_solver {
     int cur = 0;
     int *d_perm = nullptr;
     int *d_seg = nullptr, *d_nseg = nullptr;   // non-empty cell-block segments; two counts, by slab parity
+    int *d_seglen = nullptr;                // their lengths, where the block scan wrote them
     int persist_grid = 1;
     int g2p_grid = 1;
     SortScratch ws{};
@@ -85,7 +88,12 @@ struct gy_solver {
     int *skey_buf[2] = {nullptr, nullptr};  // sorted keys of the last sort and its successor
     int *d_blk_first = nullptr;             // first position of each cell block at the last sort
     int sk = 0;
-    bool resort_valid = false;              // slab order = order of the sort in skey_buf[sk]
+    bool resort_valid = false;              // slab order = order of the sort in skey_buf[sk], and every
+                                            // G2P since has flagged the movers
+    BlockSort bs{};                         // block merge sort (bs.nblk 0: the grid has too many blocks for it)
+    void *blocks_mem = nullptr;
+    int fb = 0;                             // bs.first[fb] is the last sort's
+    bool blocks_valid = false;              // slab order = that sort's, one G2P since, which kept the counts
     StepScalars *d_sc = nullptr;            // this step's scalars (device)
     static constexpr int kRing = 32;        // pinned staging slots for the per-step scalars
     StepScalars *h_ring = nullptr;
@@ -143,6 +151,18 @@ struct gy_solver {
 
 static constexpr long long kMaxTimedSteps = 4096;
 
+// The block merge sort scans every cell block of the grid in one cluster; grids with more blocks
+// (12 million particles at eight per cell fill 23,000) take the incremental re-sort, whose work
+// does not depend on the grid.
+static constexpr long long BLOCK_SORT_MAX = 1 << 20;
+
+// Particles per segment of a sorted step: whole cell blocks on large problems; pieces on small
+// ones, so that the segments, one per CTA, occupy the chip.
+static int segment_piece(long long n)
+{
+    return n >= 400000 ? 1 << 30 : n >= 100000 ? 128 : 64;
+}
+
 namespace {
 
 gy_status fail(gy_solver *h, gy_status code, const std::string &msg)
@@ -190,7 +210,7 @@ void free_device(gy_solver *h)
         h->ring_ev[k] = nullptr;
         h->ring_busy[k] = false;
     }
-    void *ptrs[] = {h->slab[0], h->slab[1], h->d_perm, h->d_seg, h->d_nseg, h->sort_mem, h->resort_mem, h->d_pbc_val,
+    void *ptrs[] = {h->slab[0], h->slab[1], h->d_perm, h->d_seg, h->d_seglen, h->blocks_mem, h->d_nseg, h->sort_mem, h->resort_mem, h->d_pbc_val,
                     h->d_refkey0, h->d_mats, h->d_status, h->d_stats, h->node_mem, h->d_cell_min,
                     h->d_nidx[0], h->d_nidx[1], h->d_nidx[2], h->d_sc, h->d_therm, h->d_tnode, h->d_tset, h->d_flaw,
                     h->d_dplog, h->d_dplog_n, h->d_pend, h->d_pend_n, h->d_surr, h->d_surr_counts};
@@ -203,7 +223,9 @@ void free_device(gy_solver *h)
     h->tset_bytes = 0;
     h->thermal = false;
     h->slab[0] = h->slab[1] = nullptr;
-    h->d_perm = h->d_seg = h->d_nseg = nullptr;
+    h->d_perm = h->d_seg = h->d_seglen = h->d_nseg = nullptr;
+    h->blocks_mem = nullptr;
+    h->bs = BlockSort{};
     h->sort_mem = nullptr;
     h->resort_mem = nullptr;
     h->skey_buf[0] = h->skey_buf[1] = nullptr;
@@ -819,7 +841,16 @@ gy_status gy_initialize(gy_solver *h, const gy_material *mats, int nmat, const g
     if ((st = dalloc(h, &h->d_perm, h->cap))) return st;
     // multi-body handles: the second half lists the segments the one-object P2G defers
     if ((st = dalloc(h, &h->d_seg, (h->multi ? 2 : 1) * h->cap))) return st;
+    if ((st = dalloc(h, &h->d_seglen, h->cap))) return st;
     if ((st = dalloc(h, &h->d_nseg, 4))) return st;
+    if (const long long nblk = (long long)h->g.nbx * h->g.nby * h->g.nbz; nblk <= BLOCK_SORT_MAX) {
+        const size_t bytes = block_sort_ints(nblk, h->cap) * sizeof(int);
+        CK(h, cudaMalloc(&h->blocks_mem, bytes));
+        CK(h, cudaMemsetAsync(h->blocks_mem, 0, bytes, h->stream));
+        block_sort_bind(h->bs, (int *)h->blocks_mem, nblk, h->cap);
+        h->fb = 0;
+    }
+    h->blocks_valid = false;
     CK(h, cudaMemsetAsync(h->d_nseg, 0, 4 * sizeof(int), h->stream));
     {
         int dev = 0, sms = 1;
@@ -918,7 +949,7 @@ static StepScalars make_scalars(const gy_solver *h, int step)
     return sc;
 }
 
-static StepArgs make_args(gy_solver *h)
+static StepArgs make_args(gy_solver *h, bool blocks)
 {
     StepArgs a{};
     a.g = h->g;
@@ -927,9 +958,17 @@ static StepArgs make_args(gy_solver *h)
     a.mats = h->d_mats;
     a.pbc_val = h->d_pbc_val;
     a.flaw = h->d_flaw;
-    // G2P flags the particles that change cell for the next incremental re-sort
-    a.mover_mask = h->rs.wmask;
-    a.mover_cnt = h->rs.wcnt;
+    // G2P notes the particles that change cell for the next sort
+    if (blocks) {
+        a.blk_cnt = h->bs.cnt;
+        a.blk_in = h->bs.in_cnt;
+        a.blk_dirty = h->bs.dirty;
+        a.mov = h->bs.mov;
+        a.mov_n = h->bs.mov_n;
+    } else {
+        a.mover_mask = h->rs.wmask;
+        a.mover_cnt = h->rs.wcnt;
+    }
     if (h->dplog_on) {
         a.dp.log_x = h->d_dplog;
         a.dp.log_y = h->d_dplog + (size_t)h->dplog_cap * 16;
@@ -950,12 +989,16 @@ static StepArgs make_args(gy_solver *h)
 // The stream work of one step (no host state changes): sort, P2G, fold + solve, G2P.
 static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
 {
-    const StepArgs a = make_args(h);
+    const StepArgs a = make_args(h, v.blocks != 0);
     cudaStream_t s = h->stream;
     if (tev) cudaEventRecord(tev[0], s);
-    // (a) stable counting sort of the cell keys; the particle kernels read through perm
+    // (a) stable sort of the cell keys; the particle kernels read through perm
     const int *perm = nullptr;
-    const int *skey = reinterpret_cast<const int *>(h->slab[v.cur]) + (size_t)PF_KEY * h->cap;
+    const int *key = reinterpret_cast<const int *>(h->slab[v.cur]) + (size_t)PF_KEY * h->cap;
+    const int *skey = key;
+    // multi-body: the one-object P2G lists the segments it leaves to the body-slot kernel
+    int *ndefer = h->multi && !h->opt.track_normals ? h->d_nseg + 2 : nullptr;
+    int *nseg = h->d_nseg + v.cur;
     if (v.sort) {
         int *out = h->skey_buf[v.sk];
         int key_bits = 1;
@@ -965,21 +1008,31 @@ static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
             // the slab is in the order of the last sort: re-sort only the particles that moved,
             // which every G2P since that sort has flagged (the mover words start clear, and
             // each re-sort clears them after use)
-            resort_keys(skey, h->skey_buf[v.sk ^ 1], out, h->d_perm, h->n, key_bits, h->rs, s, true, h->d_blk_first);
-        } else {
-            const int *sorted = sort_pairs(skey, h->d_perm, h->n, key_bits, h->ws, s);
+            resort_keys(key, h->skey_buf[v.sk ^ 1], out, h->d_perm, h->n, key_bits, h->rs, s, true, h->d_blk_first);
+        } else if (v.sort == 2) {
+            const int *sorted = sort_pairs(key, h->d_perm, h->n, key_bits, h->ws, s);
             if (h->n > 0 && sorted != out)
                 cudaMemcpyAsync(out, sorted, (size_t)h->n * sizeof(int), cudaMemcpyDeviceToDevice, s);
         }
         skey = out;
         perm = h->d_perm;
     }
-    // the segment count alternates between two counters by slab parity: this step's block
-    // heads fill one and zero the other for the next step, and zero this step's active
-    // node-block count and list length
-    int *nseg = h->d_nseg + v.cur;
-    launch_block_heads(skey, h->n, h->d_seg, nseg, s, h->nb.active_n, h->nb.active_count, h->d_nseg + (v.cur ^ 1),
-                       v.sort ? h->d_blk_first : nullptr);
+    Segs sg{h->d_seg, nullptr, nseg};
+    if (v.blocks || v.sort == 3) {
+        // a sort from scratch counts the blocks; after it G2P keeps the counts
+        if (v.sort != 3) launch_blocks_count(h->bs, skey, h->n, s);
+        launch_blocks_scan(h->bs, v.fb, segment_piece(h->n), h->d_seg, h->d_seglen, nseg, s, h->nb.active_n,
+                           h->nb.active_count, h->d_nseg + (v.cur ^ 1), ndefer);
+        if (v.sort == 3) launch_blocks_place(h->bs, key, v.fb, h->skey_buf[v.sk], h->d_perm, h->n, s);
+        sg.len = h->d_seglen;
+    } else {
+        // the segment count alternates between two counters by slab parity: this step's block
+        // heads fill one and zero the other for the next step, and zero this step's active
+        // node-block count and list length
+        launch_block_heads(skey, h->n, h->d_seg, nseg, s, h->nb.active_n, h->nb.active_count, h->d_nseg + (v.cur ^ 1),
+                           v.sort ? h->d_blk_first : nullptr);
+        if (ndefer) cudaMemsetAsync(ndefer, 0, sizeof(int), s);
+    }
     PView src = pview(h, v.cur), dst = pview(h, v.cur ^ 1);
     // body slots from the sort table of the reference's cadence (Solver.cpp:91)
     if (v.tables) {
@@ -991,17 +1044,12 @@ static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
     // heat conduction: fused into the single-body P2G, a separate pass for body slots
     const bool fused_thermal = h->thermal && !h->multi;
     // multi-body: the one-object segments take the plane-lane kernel unless normals are tracked
-    int *defer = nullptr, *ndefer = nullptr;
-    if (h->multi && !h->opt.track_normals) {
-        defer = h->d_seg + h->cap;
-        ndefer = h->d_nseg + 2;
-        cudaMemsetAsync(ndefer, 0, sizeof(int), s);
-    }
-    launch_p2g(src, perm, skey, h->n, h->d_seg, nseg, h->persist_grid, h->nb, a, s,
+    int *defer = ndefer ? h->d_seg + h->cap : nullptr;
+    launch_p2g(src, perm, skey, h->n, sg, h->persist_grid, h->nb, a, s,
                fused_thermal ? h->d_therm : nullptr, fused_thermal ? h->d_tnode : nullptr, h->opt.p2g_lanes, defer,
                ndefer);
     if (h->thermal && h->multi)
-        launch_thermal_p2g(src, h->d_therm, perm, skey, h->n, h->d_seg, nseg, h->d_tnode, a, s);
+        launch_thermal_p2g(src, h->d_therm, perm, skey, h->n, sg, h->d_tnode, a, s);
     if (tev) cudaEventRecord(tev[2], s);
     // (c) periodic fold, nodal solve, grid BCs
     launch_fold(h->nb, a, s);
@@ -1010,14 +1058,14 @@ static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
     // (d) G2P + particle BCs + update + constitutive + damage, written in sorted order, with
     // the conservation sums of the updated state (their partials zeroed by the fold)
     if (h->surr_on) cudaMemsetAsync(h->d_pend_n, 0, sizeof(unsigned int), s);
-    launch_g2p_update(src, dst, perm, skey, h->n, h->d_seg, nseg, h->g2p_grid, h->nb, a,
+    launch_g2p_update(src, dst, perm, skey, h->n, sg, h->g2p_grid, h->nb, a,
                       h->opt.track_normals != 0, h->opt.check_finite != 0, h->has_dp, s,
                       fused_thermal ? h->d_therm : nullptr, fused_thermal ? h->d_tnode : nullptr);
     if (h->surr_on)
         launch_dp_surrogate(dst, h->d_pend, h->d_pend_n, (unsigned int)h->n, h->d_mats, h->d_surr, h->d_sc, h->d_flaw,
                             h->surr_tol, h->d_surr_counts, h->d_status, s);
     if (h->thermal && h->multi)
-        launch_thermal_g2p(src, h->d_therm, perm, skey, h->n, h->d_seg, nseg, h->d_tnode, h->nb, a, s);
+        launch_thermal_g2p(src, h->d_therm, perm, skey, h->n, sg, h->d_tnode, h->nb, a, s);
     else if (h->thermal)
         launch_thermal_clear(h->nb, a, h->d_tnode, s);
     if (tev) cudaEventRecord(tev[4], s);
@@ -1040,10 +1088,13 @@ static gy_status enqueue_step(gy_solver *h, double t, int step)
         h->tev_used++;
     }
     // host decisions for this step
-    StepVariant v{h->cur, h->sk, 0, 0};
-    if (h->since_sort >= h->opt.sort_every) {
-        v.sort = (h->resort_valid && !h->opt.full_sort) ? 1 : 2;
+    StepVariant v{h->cur, h->sk, 0, 0, 0, h->fb};
+    if (h->blocks_valid || h->since_sort >= h->opt.sort_every) {
+        v.sort = h->opt.full_sort ? 2 : h->blocks_valid ? 3 : h->resort_valid ? 1 : 2;
         v.sk = h->sk ^ 1;
+        // the block merge serves the sort after exactly one G2P
+        v.blocks = h->bs.nblk > 0 && h->n > 0 && h->opt.sort_every == 1 && !h->opt.full_sort;
+        if (v.blocks || v.sort == 3) v.fb = h->fb ^ 1;
     }
     if (h->multi && ((step % 10 == 0) || step == 1 || !h->tables_valid)) v.tables = h->steps == 0 ? 2 : 1;
     // every step's scalars (dt, dt at the nodes, gravity, damping, friction, BC time) travel
@@ -1091,7 +1142,10 @@ static gy_status enqueue_step(gy_solver *h, double t, int step)
     if (v.sort) {
         h->sk = v.sk;
         h->since_sort = 0;
-        h->resort_valid = true;  // this step's G2P writes the slab in this order
+        // this step's G2P writes the slab in this order, and notes the movers for one of the two
+        h->resort_valid = !v.blocks;
+        h->blocks_valid = v.blocks != 0;
+        h->fb = v.fb;
     }
     h->since_sort++;
     if (v.tables) h->tables_valid = true;
@@ -1517,6 +1571,7 @@ gy_status gy_state_load(gy_solver *h, const void *buf, int64_t bytes)
     h->tables_valid = hd.tables_valid != 0;
     h->since_sort = 1 << 30;
     h->resort_valid = false;
+    h->blocks_valid = false;
     return sum_state(h);
 }
 

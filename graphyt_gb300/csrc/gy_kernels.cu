@@ -94,10 +94,21 @@ __device__ __forceinline__ void store_state(const PView &P, long long i, const P
 }
 
 
-// A particle whose cell key changed: its bit in the next re-sort's mover words (slot i of the
-// order this step writes), and the word's count when the bit was clear
-__device__ __forceinline__ void flag_mover(const StepArgs &a, long long i)
+// A particle whose cell key changed, in slot i of the order this step writes.  For the block merge
+// sort: its block is marked, and a particle that left it is counted and listed at its new block.
+// Else its bit in the next re-sort's mover words, and the word's count when the bit was clear.
+__device__ __forceinline__ void flag_mover(const StepArgs &a, long long i, int old_key, int key)
 {
+    if (a.blk_cnt) {
+        const int bo = old_key >> CB_SHIFT, bn = key >> CB_SHIFT;
+        a.blk_dirty[bo] = 1;
+        if (bo == bn) return;
+        atomicSub(&a.blk_cnt[bo], 1);
+        atomicAdd(&a.blk_cnt[bn], 1);
+        const int arrival = atomicAdd(&a.blk_in[bn], 1);
+        a.mov[atomicAdd(a.mov_n, 1)] = make_int4(key, (int)i, arrival, 0);
+        return;
+    }
     const unsigned bit = 1u << (i & 31);
     if (!(atomicOr(&a.mover_mask[i >> 5], bit) & bit)) atomicAdd(&a.mover_cnt[i >> 5], 1);
 }
@@ -108,14 +119,14 @@ __device__ __forceinline__ void flag_mover(const StepArgs &a, long long i)
 // bulk prefetch per field issued by thread 0.  A hint only: the window stays inside the
 // slab, and a short segment costs some L2 space, not results.
 constexpr long long PF_WINDOW = 512;
-__device__ __forceinline__ void prefetch_next_segment(const PView &P, const int *perm, const int *seg_start, int nseg,
+__device__ __forceinline__ void prefetch_next_segment(const PView &P, const int *perm, const Segs &sg, int nseg,
                                                       int next, int f0, int f1)
 {
     if (threadIdx.x != 0 || next >= nseg) return;
-    const long long s = seg_start[next];
+    const long long s = sg.start[next];
     long long j0 = perm ? (long long)perm[s] : s;
     j0 &= ~3ll;  // 16-byte aligned
-    long long len = min(PF_WINDOW, P.cap - j0);
+    long long len = min(sg.len ? min(PF_WINDOW, (long long)sg.len[next] + 3) : PF_WINDOW, P.cap - j0);
     len &= ~3ll;
     if (len <= 0) return;
     for (int f = f0; f < f1; f++)
@@ -262,7 +273,7 @@ __device__ __forceinline__ void col_pair(ColAcc &A, const float4 (*W)[PC_NP], co
 // temperature and gradient kept by insertion index in therm.
 template <bool THERMAL>
 __global__ void __launch_bounds__(PC_THREADS, GY_PC_MINB) k_p2g_cols(PView P, const int *perm, const int *skey, long long n,
-                                                         const int *seg_start, const int *nseg_ptr, int sorted,
+                                                         Segs sg, int sorted,
                                                          NodeBufs nb, GridGeom g, const float4 *therm, float2 *tnode,
                                                          const DevMaterial *mats, const StepScalars *sc)
 {
@@ -277,7 +288,7 @@ __global__ void __launch_bounds__(PC_THREADS, GY_PC_MINB) k_p2g_cols(PView P, co
     __shared__ int run_cell[PC_CH];
     __shared__ int wcount[PC_WARPS];
     __shared__ long long s_end;
-    const int nseg = *nseg_ptr;
+    const int nseg = *sg.n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;
     // lane -> (run group, jj, kk); lanes 27..31 shadow lane 26 and skip the atomics
@@ -286,9 +297,9 @@ __global__ void __launch_bounds__(PC_THREADS, GY_PC_MINB) k_p2g_cols(PView P, co
     const bool scatter_lane = lane < 27;
     const float2 z2 = make_float2(0.f, 0.f);
     for (int sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
-        prefetch_next_segment(P, perm, seg_start, nseg, sgi + gridDim.x, PF_OX, PF_S5 + 1);
-        prefetch_next_segment(P, perm, seg_start, nseg, sgi + gridDim.x, PF_RHO, PF_MASS + 1);
-        const long long start = seg_start[sgi];
+        prefetch_next_segment(P, perm, sg, nseg, sgi + gridDim.x, PF_OX, PF_S5 + 1);
+        prefetch_next_segment(P, perm, sg, nseg, sgi + gridDim.x, PF_RHO, PF_MASS + 1);
+        const long long start = sg.start[sgi], end = sg.len ? start + sg.len[sgi] : n;
         const int blk = seg_block(skey, start);
         int bx, by, bz;
         decode_block(blk, g, bx, by, bz);
@@ -301,13 +312,18 @@ __global__ void __launch_bounds__(PC_THREADS, GY_PC_MINB) k_p2g_cols(PView P, co
             if (sorted) {
                 // the segment's particles in this chunk are a prefix of it; the barriers also
                 // end the previous chunk's use of the staging arrays
-                ka = ia < n ? skey[ia] : -1;
-                kb = ib < n ? skey[ib] : -1;
-                kp = (ia < n && tid > 0) ? skey[ia - 1] : -1;
-                ja = ia < n ? perm[ia] : 0;
-                jb = ib < n ? perm[ib] : 0;
-                cnt = __syncthreads_count(ia < n && (ka >> CB_SHIFT) == blk);
-                cnt += __syncthreads_count(ib < n && (kb >> CB_SHIFT) == blk);
+                ka = ia < end ? skey[ia] : -1;
+                kb = ib < end ? skey[ib] : -1;
+                kp = (ia < end && tid > 0) ? skey[ia - 1] : -1;
+                ja = ia < end ? perm[ia] : 0;
+                jb = ib < end ? perm[ib] : 0;
+                if (sg.len) {
+                    cnt = (int)min((long long)PC_CH, end - base);
+                    __syncthreads();
+                } else {
+                    cnt = __syncthreads_count(ia < end && (ka >> CB_SHIFT) == blk);
+                    cnt += __syncthreads_count(ib < end && (kb >> CB_SHIFT) == blk);
+                }
             } else {
                 cnt = (int)min((long long)PC_CH, segment_chunk_end2(skey, n, blk, base, &s_end) - base);
                 if (2 * tid < cnt) {
@@ -530,8 +546,7 @@ __device__ __forceinline__ float2 dup2(float x) { return make_float2(x, x); }
 #endif
 template <bool MULTI, bool THERMAL = false>
 __global__ void __launch_bounds__(PP_THREADS, THERMAL ? GY_PP_MINB_TH : GY_PP_MINB)
-    k_p2g_planes(PView P, const int *perm, const int *skey, long long n, const int *seg_start, const int *nseg_ptr,
-                 int sorted, NodeBufs nb, StepArgs a, int *defer, int *ndefer, const float4 *therm = nullptr,
+    k_p2g_planes(PView P, const int *perm, const int *skey, long long n, Segs sg, int sorted, NodeBufs nb, StepArgs a, int *defer, int *ndefer, const float4 *therm = nullptr,
                  float2 *tnode = nullptr)
 {
     constexpr int TF = P2G_FIELDS + (THERMAL ? 2 : 0);  // tile fields
@@ -545,15 +560,15 @@ __global__ void __launch_bounds__(PP_THREADS, THERMAL ? GY_PP_MINB_TH : GY_PP_MI
     __shared__ long long s_end;
     const GridGeom &g = a.g;
     const int epoch = a.sc->epoch;
-    const int nseg = *nseg_ptr;
+    const int nseg = *sg.n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;
     const int grp = lane / 3, kk = lane - 3 * grp;      // lanes 30, 31: group 10, no run
     const float2 z2 = make_float2(0.f, 0.f);
     for (int sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
-        prefetch_next_segment(P, perm, seg_start, nseg, sgi + gridDim.x, PF_OX, PF_S5 + 1);
-        prefetch_next_segment(P, perm, seg_start, nseg, sgi + gridDim.x, PF_RHO, PF_MASS + 1);
-        const long long start = seg_start[sgi];
+        prefetch_next_segment(P, perm, sg, nseg, sgi + gridDim.x, PF_OX, PF_S5 + 1);
+        prefetch_next_segment(P, perm, sg, nseg, sgi + gridDim.x, PF_RHO, PF_MASS + 1);
+        const long long start = sg.start[sgi], end = sg.len ? start + sg.len[sgi] : n;
         const int blk = seg_block(skey, start);
         int bx, by, bz;
         decode_block(blk, g, bx, by, bz);
@@ -565,7 +580,7 @@ __global__ void __launch_bounds__(PP_THREADS, THERMAL ? GY_PP_MINB_TH : GY_PP_MI
             obj0 = info_obj(info0);
             tb = nb.block_body[blk];
             if ((info0 & INFO_RIGID) || (tb != obj0 && tb != -1)) {
-                if (tid == 0) defer[atomicAdd(ndefer, 1)] = (int)start;
+                if (tid == 0) defer[atomicAdd(ndefer, 1)] = sgi;
                 continue;
             }
         }
@@ -576,13 +591,18 @@ __global__ void __launch_bounds__(PP_THREADS, THERMAL ? GY_PP_MINB_TH : GY_PP_MI
             int cnt, ka = -1, kb = -1, kp = -1;
             long long ja = 0, jb = 0;
             if (sorted) {
-                ka = ia < n ? skey[ia] : -1;
-                kb = ib < n ? skey[ib] : -1;
-                kp = (ia < n && tid > 0) ? skey[ia - 1] : -1;
-                ja = ia < n ? perm[ia] : 0;
-                jb = ib < n ? perm[ib] : 0;
-                cnt = __syncthreads_count(ia < n && (ka >> CB_SHIFT) == blk);
-                cnt += __syncthreads_count(ib < n && (kb >> CB_SHIFT) == blk);
+                ka = ia < end ? skey[ia] : -1;
+                kb = ib < end ? skey[ib] : -1;
+                kp = (ia < end && tid > 0) ? skey[ia - 1] : -1;
+                ja = ia < end ? perm[ia] : 0;
+                jb = ib < end ? perm[ib] : 0;
+                if (sg.len) {
+                    cnt = (int)min((long long)PP_CH, end - base);
+                    __syncthreads();
+                } else {
+                    cnt = __syncthreads_count(ia < end && (ka >> CB_SHIFT) == blk);
+                    cnt += __syncthreads_count(ib < end && (kb >> CB_SHIFT) == blk);
+                }
             } else {
                 cnt = (int)min((long long)PP_CH, segment_chunk_end2(skey, n, blk, base, &s_end) - base);
                 if (2 * tid < cnt) {
@@ -751,7 +771,7 @@ __global__ void __launch_bounds__(PP_THREADS, THERMAL ? GY_PP_MINB_TH : GY_PP_MI
         }
         if (MULTI && dropped) {
             // another object or a rigid particle: the general kernel takes the whole segment
-            if (tid == 0) defer[atomicAdd(ndefer, 1)] = (int)start;
+            if (tid == 0) defer[atomicAdd(ndefer, 1)] = sgi;
             continue;
         }
         __syncthreads();
@@ -798,8 +818,8 @@ constexpr int MB_FIELDS = 27;                 // COM m, p(3), f(3); slot s: m, p
 constexpr int MB_NP = P2G_CH + 1;             // staged row length; odd, so rows fall in other banks
 
 __global__ void __launch_bounds__(P2G_CH) k_p2g_multi_tiled(PView P, const int *perm, const int *skey, long long n,
-                                                            const int *seg_start, const int *nseg_ptr, int sorted,
-                                                            NodeBufs nb, StepArgs a)
+                                                            Segs sg, const int *pick,
+                                                            const int *npick, int sorted, NodeBufs nb, StepArgs a)
 {
     __shared__ float tile[MB_FIELDS * PT_NODES];
     __shared__ int2 tbody[PT_NODES];
@@ -812,15 +832,16 @@ __global__ void __launch_bounds__(P2G_CH) k_p2g_multi_tiled(PView P, const int *
     __shared__ int wcount[P2G_CH / 32];
     __shared__ long long s_end;
     const GridGeom &g = a.g;
-    const int nseg = *nseg_ptr;
+    const int nseg = pick ? *npick : *sg.n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ii = lane % 3, jj = (lane / 3) % 3, kk = min(lane / 9, 2);
     const bool scatter_lane = lane < 27;
     const float grx = a.sc->gravity[0], gry = a.sc->gravity[1], grz = a.sc->gravity[2];
     const float init_vol = a.sc->init_volume;
     const int epoch = a.sc->epoch;
-    for (int sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
-        const long long start = seg_start[sgi];
+    for (int q = blockIdx.x; q < nseg; q += gridDim.x) {
+        const int sgi = pick ? pick[q] : q;
+        const long long start = sg.start[sgi], end = sg.len ? start + sg.len[sgi] : n;
         const int blk = seg_block(skey, start);
         int bx, by, bz;
         decode_block(blk, g, bx, by, bz);
@@ -855,11 +876,16 @@ __global__ void __launch_bounds__(P2G_CH) k_p2g_multi_tiled(PView P, const int *
             long long j = 0;
             const long long i = base + tid;
             if (sorted) {
-                const bool inr = i < n;
+                const bool inr = i < end;
                 kcur = inr ? skey[i] : -1;
                 kprev = (inr && tid > 0) ? skey[i - 1] : -1;
                 j = inr ? perm[i] : 0;
-                cnt = __syncthreads_count(tid < P2G_CH && inr && (kcur >> CB_SHIFT) == blk);
+                if (sg.len) {
+                    cnt = (int)min((long long)P2G_CH, end - base);
+                    __syncthreads();
+                } else {
+                    cnt = __syncthreads_count(tid < P2G_CH && inr && (kcur >> CB_SHIFT) == blk);
+                }
             } else {
                 cnt = (int)min((long long)P2G_CH, segment_chunk_end(skey, n, blk, base, P2G_CH, &s_end) - base);
                 if (tid < cnt) {
@@ -1066,8 +1092,8 @@ __global__ void __launch_bounds__(P2G_CH) k_p2g_multi_tiled(PView P, const int *
     }
 }
 
-void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, const int *seg_start,
-                const int *nseg, int persist_grid, const NodeBufs &nb, const StepArgs &a, cudaStream_t s,
+void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, const Segs &sg,
+                int persist_grid, const NodeBufs &nb, const StepArgs &a, cudaStream_t s,
                 const float4 *therm, float2 *tnode, int lanes, int *defer, int *ndefer)
 {
     if (n == 0) return;
@@ -1085,12 +1111,12 @@ void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, c
         if (lanes == 3 && defer && ndefer) {
             // the one-object segments with plane lanes, the rest (listed in defer, whose count
             // the caller zeroed) with the body-slot kernel
-            k_p2g_planes<true><<<qgrid, PP_THREADS, 0, s>>>(p, perm, skey, n, seg_start, nseg, perm ? 1 : 0, nb, a,
+            k_p2g_planes<true><<<qgrid, PP_THREADS, 0, s>>>(p, perm, skey, n, sg, perm ? 1 : 0, nb, a,
                                                              defer, ndefer);
-            k_p2g_multi_tiled<<<mgrid, P2G_CH, 0, s>>>(p, perm, skey, n, defer, ndefer, perm ? 1 : 0, nb, a);
+            k_p2g_multi_tiled<<<mgrid, P2G_CH, 0, s>>>(p, perm, skey, n, sg, defer, ndefer, perm ? 1 : 0, nb, a);
             note_launch(1);
         } else {
-            k_p2g_multi_tiled<<<mgrid, P2G_CH, 0, s>>>(p, perm, skey, n, seg_start, nseg, perm ? 1 : 0, nb, a);
+            k_p2g_multi_tiled<<<mgrid, P2G_CH, 0, s>>>(p, perm, skey, n, sg, nullptr, nullptr, perm ? 1 : 0, nb, a);
         }
     } else {
         if (therm && lanes == 3) {
@@ -1102,7 +1128,7 @@ void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, c
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_p2g_planes<false, true>, PP_THREADS, 0);
                 hgrid = sms * std::max(b, 1);
             }
-            k_p2g_planes<false, true><<<hgrid, PP_THREADS, 0, s>>>(p, perm, skey, n, seg_start, nseg, perm ? 1 : 0, nb,
+            k_p2g_planes<false, true><<<hgrid, PP_THREADS, 0, s>>>(p, perm, skey, n, sg, perm ? 1 : 0, nb,
                                                                     a, nullptr, nullptr, therm, tnode);
         } else if (therm) {
             static int tgrid = 0;  // persistent grid of the variant with heat conduction
@@ -1113,7 +1139,7 @@ void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, c
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_p2g_cols<true>, PC_THREADS, 0);
                 tgrid = sms * std::max(b, 1);
             }
-            k_p2g_cols<true><<<tgrid, PC_THREADS, 0, s>>>(p, perm, skey, n, seg_start, nseg, perm ? 1 : 0, nb, a.g,
+            k_p2g_cols<true><<<tgrid, PC_THREADS, 0, s>>>(p, perm, skey, n, sg, perm ? 1 : 0, nb, a.g,
                                                            therm, tnode, a.mats, a.sc);
         } else if (lanes == 3) {
             static int pgrid = 0;  // persistent grid of the plane-lane kernel (its own occupancy)
@@ -1124,10 +1150,10 @@ void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, c
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_p2g_planes<false>, PP_THREADS, 0);
                 pgrid = sms * std::max(b, 1);
             }
-            k_p2g_planes<false><<<pgrid, PP_THREADS, 0, s>>>(p, perm, skey, n, seg_start, nseg, perm ? 1 : 0, nb, a,
+            k_p2g_planes<false><<<pgrid, PP_THREADS, 0, s>>>(p, perm, skey, n, sg, perm ? 1 : 0, nb, a,
                                                               nullptr, nullptr);
         } else {
-            k_p2g_cols<false><<<persist_grid, PC_THREADS, 0, s>>>(p, perm, skey, n, seg_start, nseg, perm ? 1 : 0, nb,
+            k_p2g_cols<false><<<persist_grid, PC_THREADS, 0, s>>>(p, perm, skey, n, sg, perm ? 1 : 0, nb,
                                                                    a.g, nullptr, nullptr, nullptr, a.sc);
         }
     }
@@ -1970,8 +1996,7 @@ __device__ __forceinline__ void g2p_node_sums(const float4 *TV, const float2 *TA
 // rate summed with the same weights, and its temperature update, in therm by insertion index.
 template <bool HAS_DP, bool THERMAL>
 __global__ void __launch_bounds__(GY_G2P_THREADS, THERMAL ? GY_G2P_MINB_TH : GY_G2P_MINB)
-    k_g2p_tiled(PView src, PView dst, const int *perm, const int *skey, long long n, const int *seg_start,
-                const int *nseg_ptr, int sorted, NodeBufs nb, StepArgs a, int check_finite, float4 *therm,
+    k_g2p_tiled(PView src, PView dst, const int *perm, const int *skey, long long n, Segs sg, int sorted, NodeBufs nb, StepArgs a, int check_finite, float4 *therm,
                 const float2 *tnode)
 {
     constexpr int NST = G2P_NBASE + (HAS_DP ? G2P_NDP : 0);
@@ -1982,13 +2007,13 @@ __global__ void __launch_bounds__(GY_G2P_THREADS, THERMAL ? GY_G2P_MINB_TH : GY_
     __shared__ float s_st[NSTAT][GY_G2P_THREADS];
     __shared__ long long s_end;
     const GridGeom &g = a.g;
-    const int nseg = *nseg_ptr;
+    const int nseg = *sg.n;
     const int tid = threadIdx.x;
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < NSTAT; k++) s_st[k][tid] = 0.f;  // each thread's own column
     for (int sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
-        const long long start = seg_start[sgi];
+        const long long start = sg.start[sgi], end = sg.len ? start + sg.len[sgi] : n;
         const int blk = seg_block(skey, start);
         int bx, by, bz;
         decode_block(blk, g, bx, by, bz);
@@ -2029,10 +2054,15 @@ __global__ void __launch_bounds__(GY_G2P_THREADS, THERMAL ? GY_G2P_MINB_TH : GY_
             if (sorted) {
                 // the particle's key and slot are loaded together; the barrier also publishes
                 // the tile.  skey[i] is the key of particle perm[i].
-                const bool inr = i < n;
+                const bool inr = i < end;
                 key = inr ? skey[i] : -1;
                 j = inr ? perm[i] : 0;
-                cnt = __syncthreads_count(inr && (key >> CB_SHIFT) == blk);
+                if (sg.len) {
+                    cnt = (int)min((long long)blockDim.x, end - base);
+                    __syncthreads();
+                } else {
+                    cnt = __syncthreads_count(inr && (key >> CB_SHIFT) == blk);
+                }
             } else {
                 cnt = (int)min((long long)blockDim.x, segment_chunk_end(skey, n, blk, base, blockDim.x, &s_end) - base);
                 if (tid < cnt) key = skey[i];
@@ -2082,7 +2112,7 @@ __global__ void __launch_bounds__(GY_G2P_THREADS, THERMAL ? GY_G2P_MINB_TH : GY_
                 if (!g.is3d) c0[2] = 0;
                 update_after_g2p<HAS_DP>(st, c0, acc, vg, L, a, check_finite != 0, i);
                 store_state<HAS_DP>(dst, i, st);
-                if (a.mover_mask && st.key != key) flag_mover(a, i);
+                if (st.key != key && (a.mover_mask || a.blk_cnt)) flag_mover(a, i, key, st.key);
                 if (THERMAL) therm[st.pid] = make_float4(th.x + thg[3] * a.sc->dt, thg[0], thg[1], thg[2]);
                 if (a.stats) particle_stats(s_st, st);
             }
@@ -2099,8 +2129,7 @@ __global__ void __launch_bounds__(GY_G2P_THREADS, THERMAL ? GY_G2P_MINB_TH : GY_
 template <bool HAS_DP, bool NRM>
 __global__ void __launch_bounds__(GY_G2PM_THREADS, GY_G2PM_MINB) k_g2p_multi_tiled(PView src, PView dst, const int *perm,
                                                                     const int *skey, long long n,
-                                                                    const int *seg_start, const int *nseg_ptr,
-                                                                    int sorted, NodeBufs nb, StepArgs a,
+                                                                    Segs sg, int sorted, NodeBufs nb, StepArgs a,
                                                                     int check_finite)
 {
     constexpr int NST = G2P_NBASE + (HAS_DP ? G2P_NDP : 0);
@@ -2112,12 +2141,12 @@ __global__ void __launch_bounds__(GY_G2PM_THREADS, GY_G2PM_MINB) k_g2p_multi_til
     __shared__ float s_st[NSTAT][GY_G2PM_THREADS];
     __shared__ long long s_end;
     const GridGeom &g = a.g;
-    const int nseg = *nseg_ptr;
+    const int nseg = *sg.n;
     const int tid = threadIdx.x;
 #pragma unroll
     for (int k = 0; k < NSTAT; k++) s_st[k][tid] = 0.f;  // each thread's own column
     for (int sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
-        const long long start = seg_start[sgi];
+        const long long start = sg.start[sgi], end = sg.len ? start + sg.len[sgi] : n;
         const int blk = seg_block(skey, start);
         int bx, by, bz;
         decode_block(blk, g, bx, by, bz);
@@ -2180,10 +2209,15 @@ __global__ void __launch_bounds__(GY_G2PM_THREADS, GY_G2PM_MINB) k_g2p_multi_til
             long long j = 0;
             const long long i = base + tid;
             if (sorted) {
-                const bool inr = i < n;
+                const bool inr = i < end;
                 key = inr ? skey[i] : -1;
                 j = inr ? perm[i] : 0;
-                cnt = __syncthreads_count(inr && (key >> CB_SHIFT) == blk);
+                if (sg.len) {
+                    cnt = (int)min((long long)blockDim.x, end - base);
+                    __syncthreads();
+                } else {
+                    cnt = __syncthreads_count(inr && (key >> CB_SHIFT) == blk);
+                }
             } else {
                 cnt = (int)min((long long)blockDim.x, segment_chunk_end(skey, n, blk, base, blockDim.x, &s_end) - base);
                 if (tid < cnt) key = skey[i];
@@ -2279,7 +2313,7 @@ __global__ void __launch_bounds__(GY_G2PM_THREADS, GY_G2PM_MINB) k_g2p_multi_til
                 if (!g.is3d) c0[2] = 0;
                 update_after_g2p<HAS_DP>(st, c0, acc, vg, L, a, check_finite != 0, i);
                 store_state<HAS_DP>(dst, i, st);
-                if (a.mover_mask && st.key != key) flag_mover(a, i);
+                if (st.key != key && (a.mover_mask || a.blk_cnt)) flag_mover(a, i, key, st.key);
                 if (NRM) {
                     dst.f(PF_NX, i) = nrm[0];
                     dst.f(PF_NY, i) = nrm[1];
@@ -2302,7 +2336,7 @@ int g2p_blocks_per_sm(bool has_dp)
 }
 
 void launch_g2p_update(const PView &src, const PView &dst, const int *perm, const int *skey, long long n,
-                       const int *seg_start, const int *nseg, int g2p_grid, const NodeBufs &nb, const StepArgs &a,
+                       const Segs &sg, int g2p_grid, const NodeBufs &nb, const StepArgs &a,
                        bool track_normals, bool check_finite, bool has_dp, cudaStream_t s, float4 *therm,
                        const float2 *tnode)
 {
@@ -2325,13 +2359,13 @@ void launch_g2p_update(const PView &src, const PView &dst, const int *perm, cons
         }
         const unsigned mg = (unsigned)mgrid[vi];
         if (has_dp && tn)
-            k_g2p_multi_tiled<true, true><<<mg, GY_G2PM_THREADS, 0, s>>>(src, dst, perm, skey, n, seg_start, nseg, srt, nb, a, cf);
+            k_g2p_multi_tiled<true, true><<<mg, GY_G2PM_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt, nb, a, cf);
         else if (has_dp)
-            k_g2p_multi_tiled<true, false><<<mg, GY_G2PM_THREADS, 0, s>>>(src, dst, perm, skey, n, seg_start, nseg, srt, nb, a, cf);
+            k_g2p_multi_tiled<true, false><<<mg, GY_G2PM_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt, nb, a, cf);
         else if (tn)
-            k_g2p_multi_tiled<false, true><<<mg, GY_G2PM_THREADS, 0, s>>>(src, dst, perm, skey, n, seg_start, nseg, srt, nb, a, cf);
+            k_g2p_multi_tiled<false, true><<<mg, GY_G2PM_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt, nb, a, cf);
         else
-            k_g2p_multi_tiled<false, false><<<mg, GY_G2PM_THREADS, 0, s>>>(src, dst, perm, skey, n, seg_start, nseg, srt, nb, a, cf);
+            k_g2p_multi_tiled<false, false><<<mg, GY_G2PM_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt, nb, a, cf);
     } else {
         const int srt = perm ? 1 : 0;
         if (therm) {
@@ -2345,16 +2379,16 @@ void launch_g2p_update(const PView &src, const PView &dst, const int *perm, cons
                 tgrid[has_dp] = sms * std::max(b, 1);
             }
             if (has_dp)
-                k_g2p_tiled<true, true><<<tgrid[1], GY_G2P_THREADS, 0, s>>>(src, dst, perm, skey, n, seg_start, nseg, srt,
+                k_g2p_tiled<true, true><<<tgrid[1], GY_G2P_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt,
                                                                              nb, a, cf, therm, tnode);
             else
-                k_g2p_tiled<false, true><<<tgrid[0], GY_G2P_THREADS, 0, s>>>(src, dst, perm, skey, n, seg_start, nseg, srt,
+                k_g2p_tiled<false, true><<<tgrid[0], GY_G2P_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt,
                                                                               nb, a, cf, therm, tnode);
         } else if (has_dp) {
-            k_g2p_tiled<true, false><<<g2p_grid, GY_G2P_THREADS, 0, s>>>(src, dst, perm, skey, n, seg_start, nseg, srt, nb,
+            k_g2p_tiled<true, false><<<g2p_grid, GY_G2P_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt, nb,
                                                                           a, cf, nullptr, nullptr);
         } else {
-            k_g2p_tiled<false, false><<<g2p_grid, GY_G2P_THREADS, 0, s>>>(src, dst, perm, skey, n, seg_start, nseg, srt, nb,
+            k_g2p_tiled<false, false><<<g2p_grid, GY_G2P_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt, nb,
                                                                            a, cf, nullptr, nullptr);
         }
     }

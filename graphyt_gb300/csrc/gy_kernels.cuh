@@ -61,6 +61,27 @@ struct DpHooks {
     unsigned int pend_cap;
 };
 
+// The segments the particle kernels take, one CTA each: the particles [start, start + len) of one
+// cell block, in cell order.  len null: a segment ends where the block of its run does.
+struct Segs {
+    const int *start, *len;
+    const int *n;
+};
+
+// Cell-block bookkeeping of the block merge sort (gy_blocks.cu); zeroed once at allocation.
+struct BlockSort {
+    int *cnt;             // particles per cell block by their current key, kept by G2P
+    int *in_cnt;          // movers that entered each block since the last sort
+    int *dirty;           // blocks in which a particle changed cell since the last sort
+    int *first[2];        // first position of each block, of the last two sorts in turn
+    int *in_off;          // first entry of each block in in_list
+    int4 *mov;            // movers to another block: key, slot, arrival number at the block
+    int *mov_n;
+    int2 *in_list, *in_sorted;  // the movers (key, slot) grouped by new block, then also in slot order
+    int *list, *list_n;   // the non-empty blocks
+    int nblk;
+};
+
 struct StepArgs {
     GridGeom g;
     const StepScalars *sc;   // per-step scalars in device memory (one small copy per step)
@@ -73,6 +94,9 @@ struct StepArgs {
     DpHooks dp;              // learned-surrogate logging / deferral (zero when off)
     unsigned *mover_mask;    // G2P flags the slots whose key changed, one bit per slot (or null),
     int *mover_cnt;          //   with the flagged count per 32 slots, for the next re-sort
+    int *blk_cnt, *blk_in, *blk_dirty;  // or, for the block merge sort, keeps its counts and its
+    int4 *mov;                          //   list of movers (blk_cnt null: not)
+    int *mov_n;
 };
 
 // partials of the conservation sums (mass, momentum, kinetic and strain energy); the host
@@ -116,8 +140,8 @@ long long launch_count();
 // therm / tnode non-null: the single-body kernel also sums the heat conduction node fields
 // (multi-body problems run launch_thermal_p2g instead).  lanes: lanes per run of equal cell in
 // the single-body kernel without heat conduction, 3 (z-plane lanes) or 9 (x-column lanes).
-void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, const int *seg_start,
-                const int *nseg, int persist_grid, const NodeBufs &nb, const StepArgs &a, cudaStream_t s,
+void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, const Segs &sg,
+                int persist_grid, const NodeBufs &nb, const StepArgs &a, cudaStream_t s,
                 const float4 *therm = nullptr, float2 *tnode = nullptr, int lanes = 3, int *defer = nullptr,
                 int *ndefer = nullptr);
 void launch_fold(const NodeBufs &nb, const StepArgs &a, cudaStream_t s);
@@ -127,7 +151,7 @@ void launch_solve(const NodeBufs &nb, const StepArgs &a, bool keep_node_fields, 
 // therm / tnode non-null: the single-body kernel also runs the heat conduction G2P and the
 // temperature update (multi-body problems run launch_thermal_g2p instead)
 void launch_g2p_update(const PView &src, const PView &dst, const int *perm, const int *skey, long long n,
-                       const int *seg_start, const int *nseg, int g2p_grid, const NodeBufs &nb, const StepArgs &a,
+                       const Segs &sg, int g2p_grid, const NodeBufs &nb, const StepArgs &a,
                        bool track_normals, bool check_finite, bool has_dp, cudaStream_t s, float4 *therm = nullptr,
                        const float2 *tnode = nullptr);
 int g2p_blocks_per_sm(bool has_dp);
@@ -146,9 +170,9 @@ void launch_gather_slab(const float *src, float *dst, const int *perm, long long
 
 // heat conduction (gy_thermal.cu): therm = (T, grad T) per insertion index, tnode = (T, rate)
 void launch_thermal_p2g(const PView &p, const float4 *therm, const int *perm, const int *skey, long long n,
-                        const int *seg_start, const int *nseg, float2 *tnode, const StepArgs &a, cudaStream_t s);
+                        const Segs &sg, float2 *tnode, const StepArgs &a, cudaStream_t s);
 void launch_thermal_g2p(const PView &p, float4 *therm, const int *perm, const int *skey, long long n,
-                        const int *seg_start, const int *nseg, const float2 *tnode, const NodeBufs &nb,
+                        const Segs &sg, const float2 *tnode, const NodeBufs &nb,
                         const StepArgs &a, cudaStream_t s);
 void launch_thermal_clear(const NodeBufs &nb, const StepArgs &a, float2 *tnode, cudaStream_t s);
 void launch_thermal_set(float4 *therm, const int *ids, const float *T, int count, long long n, cudaStream_t s);
@@ -179,6 +203,14 @@ size_t resort_scratch_ints(long long cap);
 void resort_bind(ResortScratch &rs, int *mem, long long cap);
 void resort_keys(const int *key, const int *prev_skey, int *skey_out, int *perm_out, long long n, int key_bits,
                  ResortScratch &rs, cudaStream_t s, bool mask_ready = false, const int *blk_first = nullptr);
+// block merge sort (gy_blocks.cu)
+size_t block_sort_ints(long long nblk, long long cap);
+void block_sort_bind(BlockSort &b, int *mem, long long nblk, long long cap);
+void launch_blocks_count(const BlockSort &b, const int *skey, long long n, cudaStream_t s);
+void launch_blocks_scan(const BlockSort &b, int which, int piece, int *seg_start, int *seg_len, int *nseg, cudaStream_t s,
+                        int *clear0 = nullptr, int *clear1 = nullptr, int *clear2 = nullptr, int *clear3 = nullptr);
+void launch_blocks_place(const BlockSort &b, const int *key, int which, int *skey_out, int *perm_out, long long n,
+                         cudaStream_t s);
 // err (may be null) receives the first launch failure of the sort's kernels
 const int *sort_pairs(const int *keys_in, int *perm_out, long long n, int key_bits, SortScratch &ws, cudaStream_t s,
                       cudaError_t *err = nullptr);

@@ -44,8 +44,7 @@ __device__ __forceinline__ long long th_chunk_end(const int *skey, long long n, 
 // warp takes a run with lane k owning stencil node k and sums its particles in registers,
 // then adds two shared atomics per node; the tile is flushed with global adds.
 __global__ void __launch_bounds__(TH_THREADS) k_thermal_p2g(PView P, const float4 *therm, const int *perm,
-                                                            const int *skey, long long n, const int *seg_start,
-                                                            const int *nseg_ptr, int sorted, float2 *tnode,
+                                                            const int *skey, long long n, Segs sg, int sorted, float2 *tnode,
                                                             StepArgs a)
 {
     __shared__ float tile[2 * TT_NODES];
@@ -56,13 +55,13 @@ __global__ void __launch_bounds__(TH_THREADS) k_thermal_p2g(PView P, const float
     __shared__ int wcount[TH_THREADS / 32];
     __shared__ long long s_end;
     const GridGeom &g = a.g;
-    const int nseg = *nseg_ptr;
+    const int nseg = *sg.n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;
     const int ii = lane % 3, jj = (lane / 3) % 3, kk = min(lane / 9, 2);
     const bool scatter_lane = lane < 27;
     for (int sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
-        const long long start = seg_start[sgi];
+        const long long start = sg.start[sgi], end = sg.len ? start + sg.len[sgi] : n;
         const int blk = skey[start] >> CB_SHIFT;
         int bx, by, bz;
         decode_block(blk, g, bx, by, bz);
@@ -73,7 +72,7 @@ __global__ void __launch_bounds__(TH_THREADS) k_thermal_p2g(PView P, const float
             int cnt, kc = -1, kp = -1;
             long long j = 0;
             if (sorted) {
-                const bool inr = i < n;
+                const bool inr = i < end;
                 kc = inr ? skey[i] : -1;
                 kp = (inr && tid > 0) ? skey[i - 1] : -1;
                 j = inr ? perm[i] : 0;
@@ -164,18 +163,17 @@ __global__ void __launch_bounds__(TH_THREADS) k_thermal_p2g(PView P, const float
 // G2P of the temperature gradient and rate, and the temperature update, thread per particle
 // over the segment's node tile.
 __global__ void __launch_bounds__(TH_THREADS) k_thermal_g2p(PView P, float4 *therm, const int *perm,
-                                                            const int *skey, long long n, const int *seg_start,
-                                                            const int *nseg_ptr, int sorted, const float2 *tnode,
+                                                            const int *skey, long long n, Segs sg, int sorted, const float2 *tnode,
                                                             StepArgs a)
 {
     __shared__ float2 TN[TT_NODES];
     __shared__ long long s_end;
     const GridGeom &g = a.g;
-    const int nseg = *nseg_ptr;
+    const int nseg = *sg.n;
     const int tid = threadIdx.x;
     const float dt = a.sc->dt;
     for (int sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
-        const long long start = seg_start[sgi];
+        const long long start = sg.start[sgi], end = sg.len ? start + sg.len[sgi] : n;
         const int blk = skey[start] >> CB_SHIFT;
         int bx, by, bz;
         decode_block(blk, g, bx, by, bz);
@@ -190,7 +188,7 @@ __global__ void __launch_bounds__(TH_THREADS) k_thermal_g2p(PView P, float4 *the
             int cnt, key = 0;
             long long j = 0;
             if (sorted) {
-                const bool inr = i < n;
+                const bool inr = i < end;
                 key = inr ? skey[i] : -1;
                 j = inr ? perm[i] : 0;
                 cnt = __syncthreads_count(inr && (key >> CB_SHIFT) == blk);
@@ -275,7 +273,7 @@ int grid_of(long long work, int per_cta_threads, int cap_per_sm)
 }  // namespace
 
 void launch_thermal_p2g(const PView &p, const float4 *therm, const int *perm, const int *skey, long long n,
-                        const int *seg_start, const int *nseg, float2 *tnode, const StepArgs &a, cudaStream_t s)
+                        const Segs &sg, float2 *tnode, const StepArgs &a, cudaStream_t s)
 {
     if (n == 0) return;
     static int grid = 0;
@@ -284,12 +282,12 @@ void launch_thermal_p2g(const PView &p, const float4 *therm, const int *perm, co
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_thermal_p2g, TH_THREADS, 0);
         grid = grid_of((long long)1 << 40, 1, std::max(b, 1));
     }
-    k_thermal_p2g<<<grid, TH_THREADS, 0, s>>>(p, therm, perm, skey, n, seg_start, nseg, perm ? 1 : 0, tnode, a);
+    k_thermal_p2g<<<grid, TH_THREADS, 0, s>>>(p, therm, perm, skey, n, sg, perm ? 1 : 0, tnode, a);
     note_launch(1);
 }
 
 void launch_thermal_g2p(const PView &p, float4 *therm, const int *perm, const int *skey, long long n,
-                        const int *seg_start, const int *nseg, const float2 *tnode, const NodeBufs &nb,
+                        const Segs &sg, const float2 *tnode, const NodeBufs &nb,
                         const StepArgs &a, cudaStream_t s)
 {
     if (n == 0) return;
@@ -299,7 +297,7 @@ void launch_thermal_g2p(const PView &p, float4 *therm, const int *perm, const in
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_thermal_g2p, TH_THREADS, 0);
         grid = grid_of((long long)1 << 40, 1, std::max(b, 1));
     }
-    k_thermal_g2p<<<grid, TH_THREADS, 0, s>>>(p, therm, perm, skey, n, seg_start, nseg, perm ? 1 : 0, tnode, a);
+    k_thermal_g2p<<<grid, TH_THREADS, 0, s>>>(p, therm, perm, skey, n, sg, perm ? 1 : 0, tnode, a);
     note_launch(1);
     launch_thermal_clear(nb, a, const_cast<float2 *>(tnode), s);
 }
