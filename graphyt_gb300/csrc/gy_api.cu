@@ -156,11 +156,15 @@ static constexpr long long kMaxTimedSteps = 4096;
 // does not depend on the grid.
 static constexpr long long BLOCK_SORT_MAX = 1 << 20;
 
-// Particles per segment of a sorted step: whole cell blocks on large problems; pieces on small
-// ones, so that the segments, one per CTA, occupy the chip.
+// Particles per segment of a sorted step.  A segment is one warp's work in P2G and one CTA's in
+// G2P: pieces of cell blocks spread a small problem over the chip and even out the tail of a large
+// one, at the price of a node tile loaded and flushed per piece.  Step by piece length, 64 / 128 /
+// 256 / whole blocks: 43 / 46 / 57 / 76 us at 8,000 particles, 67 / 67 / 81 / 108 at 86,000,
+// 90 / 85 / 99 / 127 at 184,000, 164 / 154 / 169 / 157 at 730,000, 394 / 365 / 395 / 375 at 2.4
+// million.
 static int segment_piece(long long n)
 {
-    return n >= 400000 ? 1 << 30 : n >= 100000 ? 128 : 64;
+    return n >= 100000 ? 128 : 64;
 }
 
 namespace {
@@ -1017,14 +1021,17 @@ static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
         skey = out;
         perm = h->d_perm;
     }
-    Segs sg{h->d_seg, nullptr, nseg};
+    Segs sg{h->d_seg, nullptr, nseg, 0};
     if (v.blocks || v.sort == 3) {
         // a sort from scratch counts the blocks; after it G2P keeps the counts
         if (v.sort != 3) launch_blocks_count(h->bs, skey, h->n, s);
-        launch_blocks_scan(h->bs, v.fb, segment_piece(h->n), h->d_seg, h->d_seglen, nseg, s, h->nb.active_n,
-                           h->nb.active_count, h->d_nseg + (v.cur ^ 1), ndefer);
-        if (v.sort == 3) launch_blocks_place(h->bs, key, v.fb, h->skey_buf[v.sk], h->d_perm, h->n, s);
+        const int piece = segment_piece(h->n);
+        launch_blocks_scan(h->bs, v.fb, piece, nseg, s, h->nb.active_n, h->nb.active_count, h->d_nseg + (v.cur ^ 1),
+                           ndefer);
+        launch_blocks_place(h->bs, v.sort == 3 ? key : nullptr, v.fb, piece, h->d_seg, h->d_seglen, h->skey_buf[v.sk],
+                            h->d_perm, h->n, s);
         sg.len = h->d_seglen;
+        sg.most = h->n / segment_piece(h->n) + std::min<long long>(h->bs.nblk, h->n);  // full pieces and remainders
     } else {
         // the segment count alternates between two counters by slab parity: this step's block
         // heads fill one and zero the other for the next step, and zero this step's active

@@ -7,9 +7,10 @@
 // the movers, each with its arrival number at its new block.  The stable order of the new keys
 // then takes two launches:
 //   k_blocks_scan   one cluster: the blocks' first positions (a prefix sum of the counts), the
-//                   segments the particle kernels take (a block's particles, cut into pieces of at
-//                   most `piece`), the non-empty blocks, and the movers grouped by their new block;
-//   k_blocks_place  a CTA per non-empty block: the permutation and the sorted keys.  A block that
+//                   non-empty blocks, the place of each one's segments among those the particle
+//                   kernels take (a block's particles, in pieces of at most `piece`), and the
+//                   movers grouped by their new block;
+//   k_blocks_place  a CTA per non-empty block: its segments, the permutation and the sorted keys.  A block that
 //                   nothing entered, left or changed cell in is copied; the others are sorted by
 //                   (cell, old slot), a stable counting sort over their 64 cells of the movers from
 //                   lower slots, the old range and the movers from higher slots, in this order.
@@ -76,16 +77,16 @@ __device__ __forceinline__ Sums cta_scan(Sums v, Sums *wsum, Sums *total)
 }
 
 // CTAS > 1: each CTA of the cluster takes a contiguous share of the blocks; it sums the share,
-// learns the shares before its own through distributed shared memory, and scans it.  first_new
-// and the segments are written, the entering counts are cleared for the next G2P and the movers
+// learns the shares before its own through distributed shared memory, and scans it.  first_new is
+// written, the entering counts are cleared for the next G2P and the movers
 // grouped by their new block.  clear0 to clear3 (may be null): counters of the caller zeroed on
 // the way.
 // It is all latency: a grid of 125 blocks took 10 us in eight CTAs, of which the three cluster
-// barriers and the exchange were half; one CTA takes 5 us, and is the faster one up to BS_ONE
-// blocks (two tiles of BS_TILE).
+// barriers and the exchange were half; one CTA takes 3.4 us, and is the faster one up to BS_ONE
+// blocks (two tiles of BS_TILE).  54,000 blocks take 16 us in the cluster.
 template <int CTAS>
-__device__ __forceinline__ void blocks_scan(const BlockSort &b, int *first_new, int piece, int *seg_start, int *seg_len,
-                                            int *nseg, int *clear0, int *clear1, int *clear2, int *clear3)
+__device__ __forceinline__ void blocks_scan(const BlockSort &b, int *first_new, int piece, int *nseg, int *clear0,
+                                            int *clear1, int *clear2, int *clear3)
 {
     __shared__ Sums wsum[BS_WARPS];
     __shared__ Sums share;
@@ -140,11 +141,7 @@ __device__ __forceinline__ void blocks_scan(const BlockSort &b, int *first_new, 
                 o[q] = at.in;
                 if (cv[q] > 0) {
                     b.list[at.ne] = i + q;
-                    int k = at.seg;
-                    for (int p = 0; p < cv[q]; p += piece, k++) {
-                        seg_start[k] = at.n + p;
-                        seg_len[k] = min(piece, cv[q] - p);
-                    }
+                    b.seg_at[at.ne] = at.seg;
                 }
                 at = at + block_sums(cv[q], mv[q], piece);
             }
@@ -176,16 +173,14 @@ __device__ __forceinline__ void blocks_scan(const BlockSort &b, int *first_new, 
     }
 }
 __global__ void __cluster_dims__(BS_CTAS, 1, 1) __launch_bounds__(BS_THREADS)
-    k_blocks_scan(BlockSort b, int *first_new, int piece, int *seg_start, int *seg_len, int *nseg, int *clear0, int *clear1,
-                  int *clear2, int *clear3)
+    k_blocks_scan(BlockSort b, int *first_new, int piece, int *nseg, int *clear0, int *clear1, int *clear2, int *clear3)
 {
-    blocks_scan<BS_CTAS>(b, first_new, piece, seg_start, seg_len, nseg, clear0, clear1, clear2, clear3);
+    blocks_scan<BS_CTAS>(b, first_new, piece, nseg, clear0, clear1, clear2, clear3);
 }
 __global__ void __launch_bounds__(BS_THREADS)
-    k_blocks_scan_one(BlockSort b, int *first_new, int piece, int *seg_start, int *seg_len, int *nseg, int *clear0,
-                      int *clear1, int *clear2, int *clear3)
+    k_blocks_scan_one(BlockSort b, int *first_new, int piece, int *nseg, int *clear0, int *clear1, int *clear2, int *clear3)
 {
-    blocks_scan<1>(b, first_new, piece, seg_start, seg_len, nseg, clear0, clear1, clear2, clear3);
+    blocks_scan<1>(b, first_new, piece, nseg, clear0, clear1, clear2, clear3);
 }
 
 // key: the particles' keys in the old order.  A block's members are numbered movers from lower
@@ -193,12 +188,35 @@ __global__ void __launch_bounds__(BS_THREADS)
 // Members go through in rounds of BP_ROUND (a full block of eight particles per cell), BP_PER
 // consecutive warps' worth per warp, so that ranks within a warp need no barrier: a warp matches
 // its lanes' cells, and the warps' counts per cell are added up once per round.  Bound by the
-// latency of its loads; a first form with a barrier-separated count per 128 members took 28 us on
-// 2.4 million particles in nearly all of whose 4750 blocks a particle had changed cell.
+// latency of its loads: 24 us (cold caches) on 2.4 million particles in nearly all of whose 4750
+// blocks a particle had changed cell; with a barrier-separated count per 128 members it took 28,
+// with a warp per block 38.
 constexpr int BP_PER = 4;
 constexpr int BP_ROUND = BP_THREADS * BP_PER;
-__global__ void __launch_bounds__(BP_THREADS) k_blocks_place(BlockSort b, const int *key, const int *first_old,
-                                                             const int *first_new, int *skey_out, int *perm_out)
+// the segments of the block at `s` in the list (a few: written by the CTA's first threads)
+__device__ __forceinline__ void put_segments(const BlockSort &b, int s, int nf, int nc, int piece, int *seg_start,
+                                             int *seg_len)
+{
+    const int at = b.seg_at[s];
+    for (int k = threadIdx.x; (long long)k * piece < nc; k += blockDim.x) {
+        seg_start[at + k] = nf + k * piece;
+        seg_len[at + k] = min(piece, nc - k * piece);
+    }
+}
+
+// the segments alone, of an order that another sort made
+__global__ void __launch_bounds__(BP_THREADS) k_blocks_segments(BlockSort b, const int *first_new, int piece,
+                                                                int *seg_start, int *seg_len)
+{
+    for (int s = blockIdx.x; s < *b.list_n; s += gridDim.x) {
+        const int nf = first_new[b.list[s]];
+        put_segments(b, s, nf, first_new[b.list[s] + 1] - nf, piece, seg_start, seg_len);
+    }
+}
+
+__global__ void __launch_bounds__(BP_THREADS, 12) k_blocks_place(BlockSort b, const int *key, const int *first_old,
+                                                             const int *first_new, int piece, int *seg_start, int *seg_len,
+                                                             int *skey_out, int *perm_out)
 {
     __shared__ int next[64];            // next position of each cell, in the rounds after the first
     __shared__ int tot[64];             // members per cell, of blocks of more than one round
@@ -213,6 +231,7 @@ __global__ void __launch_bounds__(BP_THREADS) k_blocks_place(BlockSort b, const 
         const int nf = first_new[blk], nc = first_new[blk + 1] - nf;
         const int of = first_old[blk], oc = first_old[blk + 1] - of;
         const int io = b.in_off[blk], ic = b.in_off[blk + 1] - io;
+        put_segments(b, s, nf, nc, piece, seg_start, seg_len);
         if (!b.dirty[blk] && ic == 0) {
             for (int q = tid; q < nc; q += BP_THREADS) {
                 skey_out[nf + q] = key[of + q];
@@ -238,32 +257,29 @@ __global__ void __launch_bounds__(BP_THREADS) k_blocks_place(BlockSort b, const 
         }
         if (ic) __syncthreads();
         const int lo = n_lo, members = oc + ic;
-        auto member = [&](int m, int &slot) {  // the member's cell, -1 if it left (or none)
-            slot = 0;
+        auto cell_of = [&](int m) {  // the member's cell, -1 if it left (or none)
             if (m >= members) return -1;
-            int k;
             if (m >= lo && m < lo + oc) {
-                slot = of + m - lo;
-                k = key[slot];
+                const int k = key[of + m - lo];
                 return (k >> CB_SHIFT) == blk ? (k & 63) : -1;
             }
-            const int2 v = b.in_sorted[io + (m < lo ? m : m - oc)];
-            slot = v.y;
-            return v.x & 63;
+            return b.in_sorted[io + (m < lo ? m : m - oc)].x & 63;
+        };
+        auto slot_of = [&](int m) {  // its old slot
+            return m >= lo && m < lo + oc ? of + m - lo : b.in_sorted[io + (m < lo ? m : m - oc)].y;
         };
         const bool rounds = members > BP_ROUND;
         if (rounds) {
-            int slot;
             for (int m = tid; m < members; m += BP_THREADS) {
-                const int c = member(m, slot);
+                const int c = cell_of(m);
                 if (c >= 0) atomicAdd(&tot[c], 1);
             }
             __syncthreads();
         }
         for (int m0 = 0; m0 < members; m0 += BP_ROUND) {
-            int c[BP_PER], slot[BP_PER], r[BP_PER];
+            int c[BP_PER], r[BP_PER];
 #pragma unroll
-            for (int u = 0; u < BP_PER; u++) c[u] = member(m0 + (warp * BP_PER + u) * 32 + lane, slot[u]);
+            for (int u = 0; u < BP_PER; u++) c[u] = cell_of(m0 + (warp * BP_PER + u) * 32 + lane);
 #pragma unroll
             for (int u = 0; u < BP_PER; u++) {
                 const unsigned same = __match_any_sync(0xffffffffu, c[u]);
@@ -317,7 +333,7 @@ __global__ void __launch_bounds__(BP_THREADS) k_blocks_place(BlockSort b, const 
                 if (c[u] >= 0) {
                     const int p = wcnt[warp][c[u]] + r[u];
                     skey_out[p] = (blk << CB_SHIFT) | c[u];
-                    perm_out[p] = slot[u];
+                    perm_out[p] = slot_of(m0 + (warp * BP_PER + u) * 32 + lane);
                 }
             if (m0 + BP_ROUND < members) {
                 __syncthreads();
@@ -342,7 +358,7 @@ __global__ void __launch_bounds__(256) k_blocks_count(const int *skey, int n, in
 size_t block_sort_ints(long long nblk, long long cap)
 {
     const size_t pad = ((size_t)nblk + 8) & ~(size_t)3;
-    return 6 * pad + 16 + 4 * (size_t)cap + 2 * 2 * (size_t)cap + (size_t)std::min(nblk, cap) + 64;
+    return 6 * pad + 16 + 4 * (size_t)cap + 2 * 2 * (size_t)cap + 2 * (size_t)std::min(nblk, cap) + 64;
 }
 
 void block_sort_bind(BlockSort &b, int *mem, long long nblk, long long cap)
@@ -361,7 +377,8 @@ void block_sort_bind(BlockSort &b, int *mem, long long nblk, long long cap)
     b.mov_n = p;
     b.list_n = p + 1;
     p += 16;
-    b.list = p;
+    b.list = p; p += std::min(nblk, cap);
+    b.seg_at = p;
     b.nblk = (int)nblk;
 }
 
@@ -375,20 +392,18 @@ void launch_blocks_count(const BlockSort &b, const int *skey, long long n, cudaS
     note_launch(1);
 }
 
-void launch_blocks_scan(const BlockSort &b, int which, int piece, int *seg_start, int *seg_len, int *nseg, cudaStream_t s,
-                        int *clear0, int *clear1, int *clear2, int *clear3)
+void launch_blocks_scan(const BlockSort &b, int which, int piece, int *nseg, cudaStream_t s, int *clear0, int *clear1,
+                        int *clear2, int *clear3)
 {
     if (b.nblk <= BS_ONE)
-        launch_pdl(k_blocks_scan_one, 1, BS_THREADS, s, b, b.first[which], piece, seg_start, seg_len, nseg, clear0, clear1,
-                   clear2, clear3);
+        launch_pdl(k_blocks_scan_one, 1, BS_THREADS, s, b, b.first[which], piece, nseg, clear0, clear1, clear2, clear3);
     else
-        launch_pdl(k_blocks_scan, BS_CTAS, BS_THREADS, s, b, b.first[which], piece, seg_start, seg_len, nseg, clear0, clear1,
-                   clear2, clear3);
+        launch_pdl(k_blocks_scan, BS_CTAS, BS_THREADS, s, b, b.first[which], piece, nseg, clear0, clear1, clear2, clear3);
     note_launch(1);
 }
 
-void launch_blocks_place(const BlockSort &b, const int *key, int which, int *skey_out, int *perm_out, long long n,
-                         cudaStream_t s)
+void launch_blocks_place(const BlockSort &b, const int *key, int which, int piece, int *seg_start, int *seg_len,
+                         int *skey_out, int *perm_out, long long n, cudaStream_t s)
 {
     static int sms = 0;
     if (sms == 0) {
@@ -398,8 +413,11 @@ void launch_blocks_place(const BlockSort &b, const int *key, int which, int *ske
     }
     const long long blocks = std::min<long long>(b.nblk, n);
     const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(blocks, (long long)sms * 16));
-    launch_pdl(k_blocks_place, grid, BP_THREADS, s, b, key, (const int *)b.first[which ^ 1], (const int *)b.first[which],
-               skey_out, perm_out);
+    if (key)
+        launch_pdl(k_blocks_place, grid, BP_THREADS, s, b, key, (const int *)b.first[which ^ 1],
+                   (const int *)b.first[which], piece, seg_start, seg_len, skey_out, perm_out);
+    else
+        k_blocks_segments<<<grid, BP_THREADS, 0, s>>>(b, b.first[which], piece, seg_start, seg_len);
     note_launch(1);
 }
 

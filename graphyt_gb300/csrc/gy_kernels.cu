@@ -809,6 +809,326 @@ __global__ void __launch_bounds__(PP_THREADS, THERMAL ? GY_PP_MINB_TH : GY_PP_MI
     }
 }
 
+// P2G of a sorted step: a warp per segment, no barrier and no atomic in shared memory.
+//
+// The particles of a cell share their 27 stencil nodes, so a cell's particles are summed in
+// registers, three lanes per cell each owning a z plane of nine nodes (63 sums, packed FP32x2
+// along the fields), ten cells of a chunk side by side in a warp (2D: one plane, 32 cells).  The
+// sums then go into the warp's own 6x6x6 node tile by plain read-add-write: in one step every
+// lane adds its stencil node (i, j), so that lanes of different cells of one z layer, and of
+// different planes of one cell, hit different nodes, and the steps are separated by warp
+// barriers; only cells above one another (in sparse blocks) can collide, and those chunks add
+// layer by layer.  A node is one 16-byte word of (m, p) and one of f: 4 shared accesses per node
+// and cell instead of 7 atomics, each a compare-and-swap loop of about six instructions, which
+// were half of the kernel when every node takes weight.
+//
+// A chunk is the next ten cells' particles, at most PW_ROWS.  Staged per particle, 96 bytes: mass,
+// momentum, -V sigma / h, the end nodes' x and y weights and gradients (the middle node's follow
+// from partition of unity) and the z weight and gradient of each plane.  The f_z sums of two
+// rows are packed like the x and y components of one, so that a particle costs a lane about 140
+// instructions (190 with the weights formed by each lane from the offsets, and f_z unpacked).
+// Tile and staging take 15.8 KB, 14 warps per SM.
+//
+// MULTI, THERMAL: as in k_p2g_planes (a segment of several objects is left to `defer` before
+// anything of it is flushed).
+constexpr int PW_ROWS = 80;                          // particles of a chunk
+constexpr int PW_SROWS = PW_ROWS + PW_ROWS / 8;      // rows swizzled q + q / 8: ten cells' rows in other banks
+constexpr int PW_PLANE = PT * PT + 1;                // tile plane stride: planes in other banks
+constexpr int PW_TILE = PT * PW_PLANE;
+constexpr int PW_RUNS = 32;                          // most cells of a chunk (2D)
+
+// GIMP weights and gradients of gimp_axis without its branch: with q = max(u - (1 - l), 0) and
+// a = 2 l - q the end nodes' pieces are a^2 / 4l + max(1 - l - u, 0) and q^2 / 4l, their gradients
+// -a / 2l and q / 2l, and the middle node has the rest of 1 and of 0.
+__device__ __forceinline__ void gimp_axis_flat(float u, const GridGeom &g, float S[3], float G[3])
+{
+    const float d = u - (1.0f - g.lp);
+    const float q = fmaxf(d, 0.0f), a = 2.0f * g.lp - q;
+    S[0] = fmaf(a * g.inv_4l, a, fmaxf(-d, 0.0f));
+    S[2] = q * g.inv_4l * q;
+    S[1] = 1.0f - S[0] - S[2];
+    G[0] = -a * g.inv_2l;
+    G[2] = q * g.inv_2l;
+    G[1] = -G[0] - G[2];
+}
+
+template <bool MULTI, bool THERMAL>
+__global__ void __launch_bounds__(32, 14)
+    k_p2g_warps(PView P, const int *perm, const int *skey, Segs sg, NodeBufs nb, StepArgs a, int *defer, int *ndefer,
+                const float4 *therm, float2 *tnode)
+{
+    __shared__ float4 T0[PW_TILE], T1[PW_TILE];              // node (m, p), (f, -)
+    __shared__ float2 T2[THERMAL ? PW_TILE : 1];             // node (temperature sum, rate)
+    __shared__ float4 WX[PW_SROWS], WY[PW_SROWS];            // (S_0, S_2, G_0, G_2)
+    __shared__ float2 WZ[3][PW_SROWS];                       // (S, G) of each plane
+    __shared__ float4 R1[PW_SROWS], R2[PW_SROWS];            // (m, m v); -(s0, s3, s5, s4)
+    __shared__ float2 R3[PW_SROWS];                          // -(s1, s2)
+    __shared__ float4 R4[THERMAL ? PW_SROWS : 1];            // (T m c, -g), g = (m / rho) k grad T / h
+    __shared__ int rs[PW_RUNS + 1], rc[PW_RUNS];
+    const GridGeom &g = a.g;
+    const int epoch = a.sc->epoch;
+    const int nseg = *sg.n;
+    const int lane = threadIdx.x;
+    const unsigned lt = (1u << lane) - 1u;
+    const int planes = g.is3d ? 3 : 1, most = g.is3d ? 10 : 32;
+    const int run = g.is3d ? lane / 3 : lane, kk = g.is3d ? lane - 3 * run : 0;
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float2 z2 = make_float2(0.f, 0.f);
+    for (int sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
+        prefetch_next_segment(P, perm, sg, nseg, sgi + gridDim.x, PF_OX, PF_S5 + 1);
+        prefetch_next_segment(P, perm, sg, nseg, sgi + gridDim.x, PF_RHO, PF_MASS + 1);
+        const int start = sg.start[sgi], end = start + sg.len[sgi];
+        int key[3], slot[3];  // the chunk's keys and slots, loaded a chunk ahead
+#pragma unroll
+        for (int u = 0; u < 3; u++) {
+            const int i = start + 32 * u + lane;
+            key[u] = i < end ? skey[i] : -1;
+            slot[u] = i < end ? perm[i] : 0;
+        }
+        const int blk = __shfl_sync(0xffffffffu, key[0], 0) >> CB_SHIFT;
+        int obj0 = 0, tb = -1;
+        if (MULTI) {
+            const uint32_t info0 = (uint32_t)P.ii(PF_INFO, __shfl_sync(0xffffffffu, slot[0], 0));
+            obj0 = info_obj(info0);
+            tb = nb.block_body[blk];
+            if ((info0 & INFO_RIGID) || (tb != obj0 && tb != -1)) {
+                if (lane == 0) defer[atomicAdd(ndefer, 1)] = sgi;
+                continue;
+            }
+        }
+        for (int t = lane; t < PW_TILE; t += 32) {
+            T0[t] = T1[t] = z4;
+            if (THERMAL) T2[t] = z2;
+        }
+        bool dropped = false;
+        for (int base = start; base < end;) {
+            // ---- the chunk: whole cells, `most` of them or PW_ROWS particles at most ----
+            const int left = min(PW_ROWS, end - base);
+            unsigned heads[3];
+            bool head[3];
+#pragma unroll
+            for (int u = 0; u < 3; u++) {
+                int before = __shfl_up_sync(0xffffffffu, key[u], 1);
+                const int last = u ? __shfl_sync(0xffffffffu, key[u ? u - 1 : 0], 31) : -1;
+                if (lane == 0) before = last;
+                head[u] = 32 * u + lane < left && key[u] != before;
+                heads[u] = __ballot_sync(0xffffffffu, head[u]);
+            }
+            int cnt = left, nh = 0;
+#pragma unroll
+            for (int u = 0; u < 3; u++) {
+                const int rank = nh + __popc(heads[u] & lt);
+                if (head[u] && rank < most) {
+                    rs[rank] = 32 * u + lane;
+                    rc[rank] = key[u] & 63;
+                }
+                const unsigned past = __ballot_sync(0xffffffffu, head[u] && rank == most);
+                if (past) cnt = 32 * u + __ffs(past) - 1;
+                nh += __popc(heads[u]);
+            }
+            const int R = min(nh, most);
+            if (lane == 0) rs[R] = cnt;
+            // ---- stage its payload ----
+            bool ok = true;
+#pragma unroll
+            for (int u = 0; u < 3; u++) {
+                const int q = 32 * u + lane;
+                if (q >= cnt) break;
+                const int j = slot[u];
+                const int row = q + (q >> 3);
+                if (MULTI) {
+                    const uint32_t info = (uint32_t)P.ii(PF_INFO, j);
+                    ok = ok && !(info & INFO_RIGID) && info_obj(info) == obj0;
+                }
+                const float m = P.f(PF_MASS, j);
+                const float sc = -(m / P.f(PF_RHO, j)) * g.inv_h;  // -V sigma with the gradient's 1/h
+                float S[3], G[3];
+                gimp_axis_flat(P.f(PF_OX, j), g, S, G);
+                WX[row] = make_float4(S[0], S[2], G[0], G[2]);
+                gimp_axis_flat(P.f(PF_OY, j), g, S, G);
+                WY[row] = make_float4(S[0], S[2], G[0], G[2]);
+                if (g.is3d) {
+                    gimp_axis_flat(P.f(PF_OZ, j), g, S, G);
+                } else {
+                    S[0] = 1.f;
+                    G[0] = 0.f;
+                }
+#pragma unroll
+                for (int z = 0; z < 3; z++)
+                    if (z < planes) WZ[z][row] = make_float2(S[z], G[z]);
+                R1[row] = make_float4(m, m * P.f(PF_VX, j), m * P.f(PF_VY, j), m * P.f(PF_VZ, j));
+                R2[row] = make_float4(P.f(PF_S0, j) * sc, P.f(PF_S3, j) * sc, P.f(PF_S5, j) * sc, P.f(PF_S4, j) * sc);
+                R3[row] = make_float2(P.f(PF_S1, j) * sc, P.f(PF_S2, j) * sc);
+                if (THERMAL) {
+                    const DevMaterial &Mt = a.mats[info_mat((uint32_t)P.ii(PF_INFO, j))];
+                    const float4 th = therm[P.ii(PF_PID, j)];
+                    const float vk = sc * Mt.k_th;
+                    R4[row] = make_float4(th.x * m * Mt.c_th, vk * th.y, vk * th.z, vk * th.w);
+                }
+            }
+            if (MULTI && !__all_sync(0xffffffffu, ok)) {
+                dropped = true;
+                break;
+            }
+            base += cnt;
+            // the next chunk's keys and slots travel while this one is summed
+#pragma unroll
+            for (int u = 0; u < 3; u++) {
+                const int i = base + 32 * u + lane;
+                key[u] = i < end ? skey[i] : -1;
+                slot[u] = i < end ? perm[i] : 0;
+            }
+            __syncwarp();
+            // ---- a lane per cell and plane: the cell's particles into nine nodes' sums ----
+            const bool rv = run < R;
+            const int p0 = rv ? rs[run] : 0, len = rv ? rs[run + 1] - p0 : 0;
+            const int cell = rv ? rc[run] : 0;
+            const int maxlen = __reduce_max_sync(0xffffffffu, len);
+            float2 amp[3][3], app[3][3], afxy[3][3];  // [j][i]: (m, px), (py, pz), (fx, fy)
+            float2 afz01[3];                          // f_z of rows j = 0 and 1
+            float afz2[3];                            // f_z of row 2
+            float atT[THERMAL ? 3 : 1][3], atR[THERMAL ? 3 : 1][3];
+#pragma unroll
+            for (int j = 0; j < 3; j++)
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    amp[j][i] = app[j][i] = afxy[j][i] = z2;
+                    if (j == 0) {
+                        afz01[i] = z2;
+                        afz2[i] = 0.f;
+                    }
+                    if (THERMAL) atT[j][i] = atR[j][i] = 0.f;
+                }
+            for (int k = 0; k < maxlen; k++) {
+                const int q = p0 + min(k, max(len - 1, 0));
+                const int row = q + (q >> 3);
+                const float4 X = WX[row], Y = WY[row], D = R1[row], E = R2[row];
+                const float2 F = R3[row];
+                float2 Z = WZ[kk][row];
+                if (k >= len) Z = z2;  // past the cell's particles (or no cell): adds nothing
+                const float Sx[3] = {X.x, 1.0f - X.x - X.y, X.y}, Gx[3] = {X.z, -X.z - X.w, X.w};
+                const float Sy[3] = {Y.x, 1.0f - Y.x - Y.y, Y.y}, Gy[3] = {Y.z, -Y.z - Y.w, Y.w};
+                const float2 mvx = make_float2(D.x, D.y), mvyz = make_float2(D.z, D.w);
+                const float2 s03 = make_float2(E.x, E.y), s54 = make_float2(E.z, E.w);
+                const float2 s31 = make_float2(E.y, F.x);
+                // y and z factors, rows 0 and 1 packed
+                const float2 Sy01 = make_float2(Sy[0], Sy[1]), Gy01 = make_float2(Gy[0], Gy[1]);
+                const float2 a01 = mul2(Sy01, dup2(Z.x)), b01 = mul2(Gy01, dup2(Z.x)), c01 = mul2(Sy01, dup2(Z.y));
+                const float syz[3] = {a01.x, a01.y, Sy[2] * Z.x}, gyz[3] = {b01.x, b01.y, Gy[2] * Z.x};
+                const float syg[3] = {c01.x, c01.y, Sy[2] * Z.y};
+                // f_z: B = s5 S_y S_z, C = s4 G_y S_z + s2 S_y G_z
+                const float2 Bz01 = mul2(a01, dup2(E.z)), Cz01 = fma2(b01, dup2(E.w), mul2(c01, dup2(F.y)));
+                const float Bz2 = E.z * syz[2], Cz2 = fmaf(E.w, gyz[2], F.y * syg[2]);
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    afz01[i] = fma2(dup2(Gx[i]), Bz01, fma2(dup2(Sx[i]), Cz01, afz01[i]));
+                    afz2[i] = fmaf(Gx[i], Bz2, fmaf(Sx[i], Cz2, afz2[i]));
+                }
+                float4 TG = z4;
+                if (THERMAL) TG = R4[row];
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    const float2 syz2 = dup2(syz[j]);
+                    const float2 mp = mul2(syz2, mvx);                                    // (m, m vx) S_y S_z
+                    const float2 pp = mul2(syz2, mvyz);                                   // (m vy, m vz) S_y S_z
+                    const float2 Bxy = mul2(syz2, s03);                                   // (s0, s3) S_y S_z
+                    const float2 Cxy = fma2(dup2(gyz[j]), s31, mul2(dup2(syg[j]), s54));  // (s3, s1) G_y S_z + (s5, s4) S_y G_z
+#pragma unroll
+                    for (int i = 0; i < 3; i++) {
+                        const float2 sx = dup2(Sx[i]), gx = dup2(Gx[i]);
+                        amp[j][i] = fma2(sx, mp, amp[j][i]);
+                        app[j][i] = fma2(sx, pp, app[j][i]);
+                        afxy[j][i] = fma2(gx, Bxy, fma2(sx, Cxy, afxy[j][i]));
+                    }
+                    if (THERMAL) {
+                        const float tS = syz[j] * TG.x, Bt = TG.y * syz[j], Ct = fmaf(TG.z, gyz[j], TG.w * syg[j]);
+#pragma unroll
+                        for (int i = 0; i < 3; i++) {
+                            atT[j][i] = fmaf(Sx[i], tS, atT[j][i]);
+                            atR[j][i] = fmaf(Gx[i], Bt, fmaf(Sx[i], Ct, atR[j][i]));
+                        }
+                    }
+                }
+            }
+            // ---- into the tile, node (i, j) of every lane's plane at a time ----
+            const int lk = cell >> 4;
+            const int t0 = (lk + kk) * PW_PLANE + ((cell >> 2) & 3) * PT + (cell & 3);
+            // cells above one another in this chunk: their planes overlap
+            const unsigned column = __match_any_sync(0xffffffffu, rv ? (cell & 15) : 16 + lane);
+            const int layers = __any_sync(0xffffffffu, rv && __popc(column) > planes) ? 4 : 1;
+            for (int l = 0; l < layers; l++) {
+                const bool mine = rv && (layers == 1 || l == lk);
+#pragma unroll
+                for (int j = 0; j < 3; j++)
+#pragma unroll
+                    for (int i = 0; i < 3; i++) {
+                        const int t = t0 + j * PT + i;
+                        if (mine) {
+                            float4 A = T0[t], B = T1[t];
+                            A.x += amp[j][i].x;
+                            A.y += amp[j][i].y;
+                            A.z += app[j][i].x;
+                            A.w += app[j][i].y;
+                            B.x += afxy[j][i].x;
+                            B.y += afxy[j][i].y;
+                            B.z += j == 0 ? afz01[i].x : j == 1 ? afz01[i].y : afz2[i];
+                            T0[t] = A;
+                            T1[t] = B;
+                            if (THERMAL) {
+                                float2 C = T2[t];
+                                C.x += atT[j][i];
+                                C.y += atR[j][i];
+                                T2[t] = C;
+                            }
+                        }
+                        __syncwarp();
+                    }
+            }
+        }
+        if (MULTI && dropped) {
+            // another object or a rigid particle: the general kernel takes the whole segment
+            if (lane == 0) defer[atomicAdd(ndefer, 1)] = sgi;
+            continue;
+        }
+        // ---- flush the tile: two vector reductions per touched node ----
+        int bx, by, bz;
+        decode_block(blk, g, bx, by, bz);
+        const int tox = bx * CB, toy = by * CB, toz = g.is3d ? bz * CB : 0;
+        float grav[3] = {0.f, 0.f, 0.f};
+        if (MULTI)
+            for (int c = 0; c < 3; c++) grav[c] = __ldg(&a.sc->gravity[c]);
+        for (int t = lane; t < PW_TILE; t += 32) {
+            const float4 A = T0[t];
+            float4 B = T1[t];
+            if (A.x == 0.f && A.y == 0.f && A.z == 0.f && A.w == 0.f && B.x == 0.f && B.y == 0.f && B.z == 0.f) continue;
+            const int pl = t / PW_PLANE, r = t - pl * PW_PLANE;
+            const int ni = tox + r % PT, nj = toy + r / PT, nk = toz + pl;
+            if (ni >= g.nx || nj >= g.ny || nk >= g.nz) continue;
+            const int nd = node_index(ni, nj, nk, g);
+            if (MULTI) {
+                const bool slot0 = tb >= 0 && __ldg(&nb.body[nd].x) >= 0;
+                // the multi-body step adds gravity in P2G, as sum w m g (Extrapolation.cpp:226-278)
+                B.x += A.x * grav[0];
+                B.y += A.x * grav[1];
+                B.z += A.x * grav[2];
+                if (slot0) {
+                    red_add4(&nb.bacc0[0][nd], A.x, A.y, A.z, A.w);
+                    red_add4(&nb.bacc1[0][nd], B.x, B.y, B.z, 0.f);
+                }
+            }
+            red_add4(&nb.acc0[nd], A.x, A.y, A.z, A.w);
+            red_add4(&nb.acc1[nd], B.x, B.y, B.z, 0.f);
+            if (THERMAL) {
+                const float2 C = T2[t];
+                atomicAdd(&tnode[nd].x, C.x);
+                atomicAdd(&tnode[nd].y, C.y);
+            }
+            mark_node(nb, ni, nj, nk, g, epoch);
+        }
+        __syncwarp();
+    }
+}
+
 // Multi-body P2G through a shared-memory node tile: segments, staging and runs of equal cell
 // as in the single-body kernel, with a warp taking one run at a time (lane k = stencil node
 // k), one particle per step, and, per node, the centre-of-mass fields plus the two body
@@ -1092,11 +1412,37 @@ __global__ void __launch_bounds__(P2G_CH) k_p2g_multi_tiled(PView P, const int *
     }
 }
 
+// CTAs for at most `most` segments (0: not known), of a resident wave of `wave`
+static unsigned seg_grid(int wave, long long most) { return (unsigned)(most > 0 && most < wave ? most : wave); }
+
 void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, const Segs &sg,
                 int persist_grid, const NodeBufs &nb, const StepArgs &a, cudaStream_t s,
                 const float4 *therm, float2 *tnode, int lanes, int *defer, int *ndefer)
 {
     if (n == 0) return;
+    // a sorted step whose segments are known takes the warp kernel; 9 lanes ask for the column
+    // kernel (and on multi-body problems for the body-slot kernel throughout)
+    const bool warps = lanes == 3 && perm && sg.len;
+    if (warps && (!a.multi_body || (defer && ndefer))) {
+        static int grid[3] = {0, 0, 0};  // resident warps of the three variants
+        const int vi = a.multi_body ? 1 : therm ? 2 : 0;
+        if (grid[vi] == 0) {
+            int dev = 0, sms = 1, b = 0;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            const void *k = vi == 2 ? (const void *)k_p2g_warps<false, true>
+                          : vi == 1 ? (const void *)k_p2g_warps<true, false> : (const void *)k_p2g_warps<false, false>;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, 32, 0);
+            grid[vi] = sms * std::max(b, 1);
+        }
+        if (a.multi_body)
+            launch_step(k_p2g_warps<true, false>, seg_grid(grid[1], sg.most), 32, s, p, perm, skey, sg, nb, a, defer, ndefer, therm, tnode);
+        else if (therm)
+            launch_step(k_p2g_warps<false, true>, seg_grid(grid[2], sg.most), 32, s, p, perm, skey, sg, nb, a, defer, ndefer, therm, tnode);
+        else
+            launch_step(k_p2g_warps<false, false>, seg_grid(grid[0], sg.most), 32, s, p, perm, skey, sg, nb, a, defer, ndefer, therm, tnode);
+        note_launch(1);
+    }
     if (a.multi_body) {
         static int mgrid = 0, qgrid = 0;  // persistent grids of the two multi-body kernels
         if (mgrid == 0) {
@@ -1111,13 +1457,17 @@ void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, c
         if (lanes == 3 && defer && ndefer) {
             // the one-object segments with plane lanes, the rest (listed in defer, whose count
             // the caller zeroed) with the body-slot kernel
-            k_p2g_planes<true><<<qgrid, PP_THREADS, 0, s>>>(p, perm, skey, n, sg, perm ? 1 : 0, nb, a,
-                                                             defer, ndefer);
-            k_p2g_multi_tiled<<<mgrid, P2G_CH, 0, s>>>(p, perm, skey, n, sg, defer, ndefer, perm ? 1 : 0, nb, a);
-            note_launch(1);
+            if (!warps)
+                k_p2g_planes<true><<<qgrid, PP_THREADS, 0, s>>>(p, perm, skey, n, sg, perm ? 1 : 0, nb, a,
+                                                                 defer, ndefer);
+            launch_step(k_p2g_multi_tiled, seg_grid(mgrid, sg.most), P2G_CH, s, p, perm, skey, n, sg, (const int *)defer,
+                       (const int *)ndefer, perm ? 1 : 0, nb, a);
+            if (!warps) note_launch(1);
         } else {
             k_p2g_multi_tiled<<<mgrid, P2G_CH, 0, s>>>(p, perm, skey, n, sg, nullptr, nullptr, perm ? 1 : 0, nb, a);
         }
+    } else if (warps) {
+        return;
     } else {
         if (therm && lanes == 3) {
             static int hgrid = 0;  // persistent grid of the plane-lane variant with heat conduction
@@ -1179,7 +1529,6 @@ int p2g_blocks_per_sm()
 template <bool MULTI>
 __global__ void __launch_bounds__(256) k_fold(NodeBufs nb, GridGeom g, const StepScalars *sc, double *stats)
 {
-    pdl_prologue();
     if (stats && blockIdx.x == 0)
         for (int q = threadIdx.x; q < STATS_SLOTS * 8; q += blockDim.x) stats[q] = 0.0;
     // the representative of an orbit has every coordinate below N - 3 and one of them below 3:
@@ -1258,8 +1607,8 @@ void launch_fold(const NodeBufs &nb, const StepArgs &a, cudaStream_t s)
     const long long mx = g.nx - 3, my = g.ny - 3, mz = g.is3d ? g.nz - 3 : 1;
     const long long orbits = 3 * my * mz + (mx - 3) * 3 * mz + (g.is3d ? (mx - 3) * (my - 3) * 3 : 0);
     const unsigned grid = (unsigned)((orbits + 255) / 256);
-    if (a.multi_body) launch_pdl(k_fold<true>, grid, 256, s, nb, g, a.sc, a.stats);
-    else launch_pdl(k_fold<false>, grid, 256, s, nb, g, a.sc, a.stats);
+    if (a.multi_body) launch_step(k_fold<true>, grid, 256, s, nb, g, a.sc, a.stats);
+    else launch_step(k_fold<false>, grid, 256, s, nb, g, a.sc, a.stats);
     note_launch(1);
 }
 
@@ -1500,7 +1849,6 @@ constexpr int SOLVE_FLAGS = 4;
 // conduction clears its node fields over them).
 __global__ void __launch_bounds__(256) k_solve_single(NodeBufs nb, StepArgs a, int keep, int want_list)
 {
-    pdl_prologue();
     const GridGeom &g = a.g;
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -1588,7 +1936,6 @@ __global__ void __launch_bounds__(256) k_solve_single(NodeBufs nb, StepArgs a, i
 template <bool MULTI>
 __global__ void __launch_bounds__(256, GY_SOLVE_MINB) k_solve_multi(NodeBufs nb, StepArgs a, int keep, int want_list)
 {
-    pdl_prologue();
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nw = (int)((gridDim.x * blockDim.x) >> 5);
@@ -1624,8 +1971,8 @@ void launch_solve(const NodeBufs &nb, const StepArgs &a, bool keep_node_fields, 
     const int keep = keep_node_fields ? 1 : 0, list = want_list ? 1 : 0;
     const long long warps = a.multi_body ? 2 * a.g.nnb : a.g.nnb;
     const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>((warps + 7) / 8, (long long)sms * 16));
-    if (a.multi_body) launch_pdl(k_solve_multi<true>, grid, 256, s, nb, a, keep, list);
-    else launch_pdl(k_solve_single, grid, 256, s, nb, a, keep, list);
+    if (a.multi_body) launch_step(k_solve_multi<true>, grid, 256, s, nb, a, keep, list);
+    else launch_step(k_solve_single, grid, 256, s, nb, a, keep, list);
     note_launch(1);
 }
 
@@ -1882,14 +2229,19 @@ __device__ __forceinline__ void particle_stats(float (*col)[NT], const PState &s
     col[4][t] += 0.5f * __fdividef(st.mass, st.rho) * se;  // volume m / rho (diagnostic precision)
 }
 
+// One warp adds a column set: each lane a few threads' entries, then a shuffle sum in FP64.
 template <int NT>
 __device__ __forceinline__ void stats_cta_flush(double *out, float (*col)[NT])
 {
     __syncthreads();
-    if (threadIdx.x < NSTAT) {
+    const int lane = threadIdx.x & 31;
+    for (int q = threadIdx.x >> 5; q < NSTAT; q += NT / 32) {
         double v = 0.0;
-        for (int t = 0; t < NT; t++) v += (double)col[threadIdx.x][t];
-        atomicAdd(&out[(blockIdx.x % STATS_SLOTS) * 8 + 1 + threadIdx.x], v);
+#pragma unroll
+        for (int t = 0; t < NT; t += 32) v += (double)col[q][t + lane];
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+        if (lane == 0) atomicAdd(&out[(blockIdx.x % STATS_SLOTS) * 8 + 1 + q], v);
     }
 }
 
@@ -2119,7 +2471,7 @@ __global__ void __launch_bounds__(GY_G2P_THREADS, THERMAL ? GY_G2P_MINB_TH : GY_
             if (cnt < (int)blockDim.x) break;
         }
     }
-    if (a.stats) stats_cta_flush(a.stats, s_st);
+    if (a.stats && (int)blockIdx.x < nseg) stats_cta_flush(a.stats, s_st);  // a CTA without a segment adds nothing
 }
 
 // Multi-body G2P + update through a shared-memory node tile: per node the body pair (or
@@ -2324,7 +2676,7 @@ __global__ void __launch_bounds__(GY_G2PM_THREADS, GY_G2PM_MINB) k_g2p_multi_til
             if (cnt < (int)blockDim.x) break;
         }
     }
-    if (a.stats) stats_cta_flush(a.stats, s_st);
+    if (a.stats && (int)blockIdx.x < nseg) stats_cta_flush(a.stats, s_st);  // a CTA without a segment adds nothing
 }
 
 int g2p_blocks_per_sm(bool has_dp)
@@ -2357,15 +2709,15 @@ void launch_g2p_update(const PView &src, const PView &dst, const int *perm, cons
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, GY_G2PM_THREADS, 0);
             mgrid[vi] = sms * std::max(b, 1);
         }
-        const unsigned mg = (unsigned)mgrid[vi];
+        const unsigned mg = seg_grid(mgrid[vi], sg.most);
         if (has_dp && tn)
-            k_g2p_multi_tiled<true, true><<<mg, GY_G2PM_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt, nb, a, cf);
+            launch_step(k_g2p_multi_tiled<true, true>, mg, GY_G2PM_THREADS, s, src, dst, perm, skey, n, sg, srt, nb, a, cf);
         else if (has_dp)
-            k_g2p_multi_tiled<true, false><<<mg, GY_G2PM_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt, nb, a, cf);
+            launch_step(k_g2p_multi_tiled<true, false>, mg, GY_G2PM_THREADS, s, src, dst, perm, skey, n, sg, srt, nb, a, cf);
         else if (tn)
-            k_g2p_multi_tiled<false, true><<<mg, GY_G2PM_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt, nb, a, cf);
+            launch_step(k_g2p_multi_tiled<false, true>, mg, GY_G2PM_THREADS, s, src, dst, perm, skey, n, sg, srt, nb, a, cf);
         else
-            k_g2p_multi_tiled<false, false><<<mg, GY_G2PM_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt, nb, a, cf);
+            launch_step(k_g2p_multi_tiled<false, false>, mg, GY_G2PM_THREADS, s, src, dst, perm, skey, n, sg, srt, nb, a, cf);
     } else {
         const int srt = perm ? 1 : 0;
         if (therm) {
@@ -2379,17 +2731,17 @@ void launch_g2p_update(const PView &src, const PView &dst, const int *perm, cons
                 tgrid[has_dp] = sms * std::max(b, 1);
             }
             if (has_dp)
-                k_g2p_tiled<true, true><<<tgrid[1], GY_G2P_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt,
-                                                                             nb, a, cf, therm, tnode);
+                launch_step(k_g2p_tiled<true, true>, seg_grid(tgrid[1], sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n,
+                           sg, srt, nb, a, cf, therm, tnode);
             else
-                k_g2p_tiled<false, true><<<tgrid[0], GY_G2P_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt,
-                                                                              nb, a, cf, therm, tnode);
+                launch_step(k_g2p_tiled<false, true>, seg_grid(tgrid[0], sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n,
+                           sg, srt, nb, a, cf, therm, tnode);
         } else if (has_dp) {
-            k_g2p_tiled<true, false><<<g2p_grid, GY_G2P_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt, nb,
-                                                                          a, cf, nullptr, nullptr);
+            launch_step(k_g2p_tiled<true, false>, seg_grid(g2p_grid, sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n, sg,
+                       srt, nb, a, cf, (float4 *)nullptr, (const float2 *)nullptr);
         } else {
-            k_g2p_tiled<false, false><<<g2p_grid, GY_G2P_THREADS, 0, s>>>(src, dst, perm, skey, n, sg, srt, nb,
-                                                                           a, cf, nullptr, nullptr);
+            launch_step(k_g2p_tiled<false, false>, seg_grid(g2p_grid, sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n, sg,
+                       srt, nb, a, cf, (float4 *)nullptr, (const float2 *)nullptr);
         }
     }
     note_launch(1);
