@@ -56,8 +56,6 @@ struct gy_solver {
     std::vector<int> mat, obj, pbc_type;
     std::vector<double> pbc_val;
     std::vector<unsigned char> hold;
-    std::vector<int> key0;           // uploaded cell key by particle id
-    std::vector<float> off0;         // uploaded FP32 offsets by particle id (3 per particle)
     std::vector<unsigned char> nbc_type;
     std::vector<float> nbc_val;
     bool any_node_bc = false;
@@ -120,6 +118,7 @@ struct gy_solver {
     float surr_tol = 1e-4f;
     bool surr_on = false;
     int *d_refkey0 = nullptr;
+    void *d_first = nullptr;                // as uploaded, by insertion index: positions, offsets, cell keys
     DevMaterial *d_mats = nullptr;
     int *d_status = nullptr;
     double *d_stats = nullptr;              // STATS_SLOTS x 8 conservation partials
@@ -215,7 +214,7 @@ void free_device(gy_solver *h)
         h->ring_busy[k] = false;
     }
     void *ptrs[] = {h->slab[0], h->slab[1], h->d_perm, h->d_seg, h->d_seglen, h->blocks_mem, h->d_nseg, h->sort_mem, h->resort_mem, h->d_pbc_val,
-                    h->d_refkey0, h->d_mats, h->d_status, h->d_stats, h->node_mem, h->d_cell_min,
+                    h->d_refkey0, h->d_first, h->d_mats, h->d_status, h->d_stats, h->node_mem, h->d_cell_min,
                     h->d_nidx[0], h->d_nidx[1], h->d_nidx[2], h->d_sc, h->d_therm, h->d_tnode, h->d_tset, h->d_flaw,
                     h->d_dplog, h->d_dplog_n, h->d_pend, h->d_pend_n, h->d_surr, h->d_surr_counts};
     for (void *p : ptrs)
@@ -246,6 +245,7 @@ void free_device(gy_solver *h)
     h->d_surr_counts = nullptr;
     h->surr_on = false;
     h->d_refkey0 = nullptr;
+    h->d_first = nullptr;
     h->d_mats = nullptr;
     h->d_status = nullptr;
     h->d_stats = nullptr;
@@ -731,8 +731,6 @@ gy_status gy_initialize(gy_solver *h, const gy_material *mats, int nmat, const g
     }
     std::vector<float> hs(slab_floats, 0.0f);
     std::vector<int> refkey0(h->cap, 0);
-    h->key0.assign((size_t)n, 0);
-    h->off0.assign((size_t)n * 3, 0.0f);
     std::vector<float4> pbcv(h->cap, make_float4(0.f, 0.f, 0.f, 0.f));
     auto F = [&](int f, long long i) -> float & { return hs[(size_t)f * h->cap + i]; };
     auto I = [&](int f, long long i) -> int & { return reinterpret_cast<int *>(hs.data())[(size_t)f * h->cap + i]; };
@@ -760,8 +758,6 @@ gy_status gy_initialize(gy_solver *h, const gy_material *mats, int nmat, const g
             F(PF_OX + a, i) = (float)off;
         }
         I(PF_KEY, i) = encode_key(c[0], c[1], h->g.is3d ? c[2] : 0, h->g);
-        h->key0[i] = I(PF_KEY, i);
-        for (int a = 0; a < 3; a++) h->off0[3 * i + a] = F(PF_OX + a, i);
         for (int k = 0; k < 3; k++) F(PF_VX + k, i) = (float)h->vel[3 * i + k];
         for (int k = 0; k < 6; k++) F(PF_S0 + k, i) = (float)h->stress[6 * i + k];
         const gy_material &M = mats[h->mat[i]];
@@ -787,6 +783,16 @@ gy_status gy_initialize(gy_solver *h, const gy_material *mats, int nmat, const g
     CK(h, cudaMemcpyAsync(h->slab[0], hs.data(), slab_floats * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     h->cur = 0;
     gy_status st;
+    // what the position and displacement getters measure from
+    CK(h, cudaMalloc(&h->d_first, (size_t)h->cap * (3 * sizeof(double) + 3 * sizeof(float) + sizeof(int))));
+    {
+        double *p0 = static_cast<double *>(h->d_first);
+        float *o0 = reinterpret_cast<float *>(p0 + 3 * h->cap);
+        CK(h, cudaMemcpyAsync(p0, h->pos.data(), (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+        CK(h, cudaMemcpyAsync(o0, h->slab[0], (size_t)h->cap * 3 * sizeof(float), cudaMemcpyDeviceToDevice, h->stream));
+        CK(h, cudaMemcpyAsync(o0 + 3 * h->cap, h->slab[0] + (size_t)PF_KEY * h->cap, (size_t)h->cap * sizeof(int),
+                              cudaMemcpyDeviceToDevice, h->stream));
+    }
     if ((st = dalloc(h, &h->d_pbc_val, h->cap))) return st;
     CK(h, cudaMemcpyAsync(h->d_pbc_val, pbcv.data(), h->cap * sizeof(float4), cudaMemcpyHostToDevice, h->stream));
     if (std::any_of(h->flaw.begin(), h->flaw.end(), [](double w) { return w != 1.0; })) {
@@ -1208,12 +1214,32 @@ gy_status gy_num_particles(const gy_solver *h, int64_t *n)
     return GY_OK;
 }
 
-static gy_status fetch_slab(gy_solver *h, std::vector<float> &hs)
+static ExportArgs export_args(const gy_solver *h)
 {
-    cudaSetDevice(h->device);
-    hs.resize((size_t)PF_COUNT * h->cap);
+    ExportArgs a{};
+    a.g = h->g;
+    a.pos0 = static_cast<const double *>(h->d_first);
+    a.off0 = reinterpret_cast<const float *>(a.pos0 + 3 * h->cap);
+    a.key0 = reinterpret_cast<const int *>(a.off0 + 3 * h->cap);
+    a.h = h->h;
+    a.init_volume = h->g.is3d ? h->psep * h->psep * h->psep : h->psep * h->psep;
+    a.has_dp = h->has_dp;
+    a.normals = h->opt.track_normals != 0;
+    for (int k = 0; k < h->nbody; k++) a.slot_obj[k] = h->slot_obj[k];
+    return a;
+}
+
+// The rows of a getter are put together in the slab the next step writes: at most 48 bytes per
+// particle at its head, where that step's G2P writes all 92 bytes of the fields up to PF_PID anew.
+static_assert(PF_PID < PF_EQPS && (PF_PID + 1) * 4 >= 6 * 8, "the getters' rows must fit the fields every step writes");
+static void *export_rows(gy_solver *h) { return h->slab[h->cur ^ 1]; }
+
+static gy_status copy_rows(gy_solver *h, void *out, size_t bytes)
+{
+    const cudaError_t le = cudaGetLastError();
+    if (le != cudaSuccess) return fail(h, GY_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(le));
+    if (bytes) CK(h, cudaMemcpyAsync(out, export_rows(h), bytes, cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
-    CK(h, cudaMemcpy(hs.data(), h->slab[h->cur], hs.size() * sizeof(float), cudaMemcpyDeviceToHost));
     return GY_OK;
 }
 
@@ -1243,73 +1269,19 @@ gy_status gy_get_particles(gy_solver *h, int field, double *out, int64_t count)
         }
         return GY_OK;
     }
+    cudaSetDevice(h->device);
     if (field == GY_P_TEMP || field == GY_P_TEMPGRAD) {
         // kept by insertion index; without a device copy every temperature is the host value
         // and every gradient zero
-        std::vector<float4> th;
-        if (h->d_therm) {
-            th.resize((size_t)n);
-            cudaSetDevice(h->device);
-            CK(h, cudaStreamSynchronize(h->stream));
-            CK(h, cudaMemcpy(th.data(), h->d_therm, (size_t)n * sizeof(float4), cudaMemcpyDeviceToHost));
+        if (!h->d_therm) {
+            for (long long i = 0; i < n * w; i++) out[i] = field == GY_P_TEMP ? h->temp[i] : 0.0;
+            return GY_OK;
         }
-        for (long long i = 0; i < n; i++) {
-            if (field == GY_P_TEMP) {
-                out[i] = h->d_therm ? (double)th[i].x : h->temp[i];
-            } else {
-                out[3 * i] = h->d_therm ? (double)th[i].y : 0.0;
-                out[3 * i + 1] = h->d_therm ? (double)th[i].z : 0.0;
-                out[3 * i + 2] = h->d_therm ? (double)th[i].w : 0.0;
-            }
-        }
-        return GY_OK;
+        launch_export_therm(h->d_therm, n, field, static_cast<double *>(export_rows(h)), h->stream);
+    } else {
+        launch_export(pview(h, h->cur), n, field, export_args(h), static_cast<double *>(export_rows(h)), h->stream);
     }
-    std::vector<float> hs;
-    gy_status st = fetch_slab(h, hs);
-    if (st) return st;
-    auto F = [&](int f, long long i) { return hs[(size_t)f * h->cap + i]; };
-    auto I = [&](int f, long long i) { return reinterpret_cast<const int *>(hs.data())[(size_t)f * h->cap + i]; };
-    const double hh = h->h;
-    for (long long i = 0; i < n; i++) {
-        const long long pid = I(PF_PID, i);
-        double *o = out + (size_t)pid * w;
-        const uint32_t info = (uint32_t)I(PF_INFO, i);
-        switch (field) {
-        case GY_P_POS:
-        case GY_P_DISP: {
-            // displacement from the change of (cell, FP32 offset) since upload, so that a
-            // particle that has not moved reports exactly zero; position = pos0 + disp
-            int c[3], c0[3];
-            auto split = [&](int key, int *cc) { decode_key(key, h->g, cc[0], cc[1], cc[2]); };
-            split(I(PF_KEY, i), c);
-            split(h->key0[pid], c0);
-            for (int k = 0; k < 3; k++) {
-                double d = 0.0;
-                if (k < 2 || h->g.is3d)
-                    d = ((double)(c[k] - c0[k]) + ((double)F(PF_OX + k, i) - (double)h->off0[3 * pid + k])) * hh;
-                o[k] = field == GY_P_POS ? h->pos[3 * pid + k] + d : d;
-            }
-            break;
-        }
-        case GY_P_POS0: for (int k = 0; k < 3; k++) o[k] = h->pos[3 * pid + k]; break;
-        case GY_P_VEL: for (int k = 0; k < 3; k++) o[k] = F(PF_VX + k, i); break;
-        case GY_P_STRESS: for (int k = 0; k < 6; k++) o[k] = F(PF_S0 + k, i); break;
-        case GY_P_STRAIN: for (int k = 0; k < 6; k++) o[k] = F(PF_E0 + k, i); break;
-        case GY_P_PSTRAIN: for (int k = 0; k < 6; k++) o[k] = h->has_dp ? F(PF_EP0 + k, i) : 0.0; break;
-        case GY_P_EQPS: o[0] = h->has_dp ? F(PF_EQPS, i) : 0.0; break;
-        case GY_P_DAMAGE: o[0] = h->has_dp ? F(PF_DMG, i) : 0.0; break;
-        case GY_P_SMAX: o[0] = h->has_dp ? F(PF_SMAX, i) : 0.0; break;
-        case GY_P_MASS: o[0] = F(PF_MASS, i); break;
-        case GY_P_DENSITY: o[0] = F(PF_RHO, i); break;
-        case GY_P_VOLUME:
-            o[0] = (info & INFO_INIT_VOL) ? (h->g.is3d ? h->psep * h->psep * h->psep : h->psep * h->psep)
-                                          : (double)F(PF_MASS, i) / (double)F(PF_RHO, i);
-            break;
-        case GY_P_NORMALS: for (int k = 0; k < 3; k++) o[k] = h->opt.track_normals ? F(PF_NX + k, i) : 0.0; break;
-        default: break;
-        }
-    }
-    return GY_OK;
+    return copy_rows(h, out, (size_t)count * sizeof(double));
 }
 
 gy_status gy_get_particles_int(gy_solver *h, int field, int *out, int64_t count)
@@ -1330,37 +1302,10 @@ gy_status gy_get_particles_int(gy_solver *h, int field, int *out, int64_t count)
         }
         return GY_OK;
     }
-    std::vector<float> hs;
-    gy_status st = fetch_slab(h, hs);
-    if (st) return st;
-    auto F = [&](int f, long long i) { return hs[(size_t)f * h->cap + i]; };
-    auto I = [&](int f, long long i) { return reinterpret_cast<const int *>(hs.data())[(size_t)f * h->cap + i]; };
-    for (long long i = 0; i < n; i++) {
-        const long long pid = I(PF_PID, i);
-        const uint32_t info = (uint32_t)I(PF_INFO, i);
-        switch (field) {
-        case GY_PI_MATERIAL: out[pid] = info_mat(info); break;
-        case GY_PI_OBJECT: out[pid] = h->slot_obj[info_obj(info)]; break;
-        case GY_PI_DEVICE_SLOT: out[pid] = (int)i; break;
-        case GY_PI_CELLID: {
-            if (info & INFO_INIT_VOL) {
-                // no update yet: the initial unshifted key (MaterialPoints.cpp:228-231)
-                const int ix = (int)(h->pos[3 * pid] / h->h), iy = (int)(h->pos[3 * pid + 1] / h->h),
-                          iz = (int)(h->pos[3 * pid + 2] / h->h);
-                out[pid] = ix + iy * (h->nx - 1) + iz * (h->nx - 1) * (h->ny - 1);
-                break;
-            }
-            int c[3];
-            decode_key(I(PF_KEY, i), h->g, c[0], c[1], c[2]);
-            int id[3] = {0, 0, 0};
-            for (int k = 0; k < (h->g.is3d ? 3 : 2); k++) id[k] = (int)((c[k] + (double)F(PF_OX + k, i)) - 0.25);
-            out[pid] = id[0] + id[1] * (h->nx - 1) + id[2] * (h->nx - 1) * (h->ny - 1);
-            break;
-        }
-        default: return GY_ERR_ARG;
-        }
-    }
-    return GY_OK;
+    if (field < GY_PI_CELLID || field > GY_PI_DEVICE_SLOT) return GY_ERR_ARG;
+    cudaSetDevice(h->device);
+    launch_export_int(pview(h, h->cur), n, field, export_args(h), static_cast<int *>(export_rows(h)), h->stream);
+    return copy_rows(h, out, (size_t)count * sizeof(int));
 }
 
 gy_status gy_get_nodes(gy_solver *h, int field, double *out, int64_t count)

@@ -225,6 +225,19 @@ void launch_blocks_scan(const BlockSort &b, int which, int piece, int *nseg, cud
 // key null: another sort has made the order, only the segments are written
 void launch_blocks_place(const BlockSort &b, const int *key, int which, int piece, int *seg_start, int *seg_len,
                          int *skey_out, int *perm_out, long long n, cudaStream_t s);
+// particle fields in insertion order and FP64 (gy_export.cu)
+struct ExportArgs {
+    GridGeom g;
+    const double *pos0;      // 3 per particle, by insertion index
+    const int *key0;         // the cell key and the offsets (field by field) a particle was uploaded with
+    const float *off0;
+    double h, init_volume;
+    bool has_dp, normals;
+    int slot_obj[MAX_BODIES];
+};
+void launch_export(const PView &p, long long n, int field, const ExportArgs &a, double *out, cudaStream_t s);
+void launch_export_int(const PView &p, long long n, int field, const ExportArgs &a, int *out, cudaStream_t s);
+void launch_export_therm(const float4 *therm, long long n, int field, double *out, cudaStream_t s);
 // err (may be null) receives the first launch failure of the sort's kernels
 const int *sort_pairs(const int *keys_in, int *perm_out, long long n, int key_bits, SortScratch &ws, cudaStream_t s,
                       cudaError_t *err = nullptr);
