@@ -93,14 +93,15 @@ struct gy_solver {
     int fb = 0;                             // bs.first[fb] is the last sort's
     bool blocks_valid = false;              // slab order = that sort's, one G2P since, which kept the counts
     StepScalars *d_sc = nullptr;            // this step's scalars (device)
-    static constexpr int kRing = 32;        // pinned staging slots for the per-step scalars
+    int *d_taken = nullptr;                 // the ring slot the next step takes
+    static constexpr int kRing = ScalarRing::SLOTS, kGroup = 8;
     StepScalars *h_ring = nullptr;
     struct Readback {
         double part[STATS_SLOTS * 8];
         int flags[4];
     } *h_rb = nullptr;                      // pinned: the step's sums and status words
-    cudaEvent_t ring_ev[kRing] = {};
-    bool ring_busy[kRing] = {};
+    cudaEvent_t ring_ev[kRing / kGroup] = {};  // the last step that reads each group of slots is done
+    bool ring_busy[kRing / kGroup] = {};
     long long ring_pos = 0;
     std::vector<StepGraph> graphs;          // captured steps, one per StepVariant
     float4 *d_pbc_val = nullptr;
@@ -208,13 +209,13 @@ void free_device(gy_solver *h)
     h->h_ring = nullptr;
     if (h->h_rb) cudaFreeHost(h->h_rb);
     h->h_rb = nullptr;
-    for (int k = 0; k < gy_solver::kRing; k++) {
+    for (int k = 0; k < gy_solver::kRing / gy_solver::kGroup; k++) {
         if (h->ring_ev[k]) cudaEventDestroy(h->ring_ev[k]);
         h->ring_ev[k] = nullptr;
         h->ring_busy[k] = false;
     }
     void *ptrs[] = {h->slab[0], h->slab[1], h->d_perm, h->d_seg, h->d_seglen, h->blocks_mem, h->d_nseg, h->sort_mem, h->resort_mem, h->d_pbc_val,
-                    h->d_refkey0, h->d_first, h->d_mats, h->d_status, h->d_stats, h->node_mem, h->d_cell_min,
+                    h->d_refkey0, h->d_first, h->d_mats, h->d_stats, h->node_mem, h->d_cell_min,
                     h->d_nidx[0], h->d_nidx[1], h->d_nidx[2], h->d_sc, h->d_therm, h->d_tnode, h->d_tset, h->d_flaw,
                     h->d_dplog, h->d_dplog_n, h->d_pend, h->d_pend_n, h->d_surr, h->d_surr_counts};
     for (void *p : ptrs)
@@ -810,13 +811,17 @@ gy_status gy_initialize(gy_solver *h, const gy_material *mats, int nmat, const g
     for (int i = 0; i < nmat; i++) dm[i] = to_dev(mats[i]);
     if ((st = dalloc(h, &h->d_mats, nmat))) return st;
     CK(h, cudaMemcpyAsync(h->d_mats, dm.data(), nmat * sizeof(DevMaterial), cudaMemcpyHostToDevice, h->stream));
-    if ((st = dalloc(h, &h->d_status, 4))) return st;
+    // the sums and the status words side by side: one copy reads both
+    if ((st = dalloc(h, &h->d_stats, STATS_SLOTS * 8 + 2))) return st;
+    h->d_status = reinterpret_cast<int *>(h->d_stats + STATS_SLOTS * 8);
     CK(h, cudaMemsetAsync(h->d_status, 0, 4 * sizeof(int), h->stream));
-    if ((st = dalloc(h, &h->d_stats, STATS_SLOTS * 8))) return st;
-    CK(h, cudaMalloc(&h->d_sc, sizeof(StepScalars)));
+    CK(h, cudaMalloc(&h->d_sc, sizeof(StepScalars) + sizeof(int)));
+    h->d_taken = reinterpret_cast<int *>(h->d_sc + 1);
+    CK(h, cudaMemsetAsync(h->d_taken, 0, sizeof(int), h->stream));
+    h->ring_pos = 0;
     CK(h, cudaMallocHost(&h->h_ring, gy_solver::kRing * sizeof(StepScalars)));
     CK(h, cudaMallocHost(&h->h_rb, sizeof(gy_solver::Readback)));
-    for (int k = 0; k < gy_solver::kRing; k++) CK(h, cudaEventCreateWithFlags(&h->ring_ev[k], cudaEventDisableTiming));
+    for (int k = 0; k < gy_solver::kRing / gy_solver::kGroup; k++) CK(h, cudaEventCreateWithFlags(&h->ring_ev[k], cudaEventDisableTiming));
     // sort scratch
     h->sort_mem = nullptr;
     const size_t sbytes = sort_scratch_bytes(h->cap);
@@ -1028,11 +1033,12 @@ static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
         perm = h->d_perm;
     }
     Segs sg{h->d_seg, nullptr, nseg, 0};
+    const ScalarRing ring{h->h_ring, h->d_taken, h->d_sc};
     if (v.blocks || v.sort == 3) {
         // a sort from scratch counts the blocks; after it G2P keeps the counts
         if (v.sort != 3) launch_blocks_count(h->bs, skey, h->n, s);
         const int piece = segment_piece(h->n);
-        launch_blocks_scan(h->bs, v.fb, piece, nseg, s, h->nb.active_n, h->nb.active_count, h->d_nseg + (v.cur ^ 1),
+        launch_blocks_scan(h->bs, ring, v.fb, piece, nseg, s, h->nb.active_n, h->nb.active_count, h->d_nseg + (v.cur ^ 1),
                            ndefer);
         launch_blocks_place(h->bs, v.sort == 3 ? key : nullptr, v.fb, piece, h->d_seg, h->d_seglen, h->skey_buf[v.sk],
                             h->d_perm, h->n, s);
@@ -1042,6 +1048,7 @@ static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
         // the segment count alternates between two counters by slab parity: this step's block
         // heads fill one and zero the other for the next step, and zero this step's active
         // node-block count and list length
+        launch_take_scalars(ring, s);
         launch_block_heads(skey, h->n, h->d_seg, nseg, s, h->nb.active_n, h->nb.active_count, h->d_nseg + (v.cur ^ 1),
                            v.sort ? h->d_blk_first : nullptr);
         if (ndefer) cudaMemsetAsync(ndefer, 0, sizeof(int), s);
@@ -1110,19 +1117,14 @@ static gy_status enqueue_step(gy_solver *h, double t, int step)
         if (v.blocks || v.sort == 3) v.fb = h->fb ^ 1;
     }
     if (h->multi && ((step % 10 == 0) || step == 1 || !h->tables_valid)) v.tables = h->steps == 0 ? 2 : 1;
-    // every step's scalars (dt, dt at the nodes, gravity, damping, friction, BC time) travel
-    // host-to-device through a pinned ring slot, ahead of the step's kernels on its stream; a
-    // slot is rewritten only after the copy that last read it has run (the host waits only
-    // when 32 steps are queued)
-    {
-        const int slot = (int)(h->ring_pos++ % gy_solver::kRing);
-        if (h->ring_busy[slot]) CK(h, cudaEventSynchronize(h->ring_ev[slot]));
-        h->epoch = h->epoch == 0x7fffffff ? 1 : h->epoch + 1;
-        h->h_ring[slot] = make_scalars(h, step);
-        CK(h, cudaMemcpyAsync(h->d_sc, &h->h_ring[slot], sizeof(StepScalars), cudaMemcpyHostToDevice, s));
-        CK(h, cudaEventRecord(h->ring_ev[slot], s));
-        h->ring_busy[slot] = true;
-    }
+    // every step's scalars (dt, dt at the nodes, gravity, damping, friction, BC time) lie in a
+    // pinned ring slot that the step's first kernel takes; a slot is rewritten only after the step
+    // that read it last is done, known by the group of slots (the host waits only when about 32
+    // steps are queued)
+    const int slot = (int)(h->ring_pos % gy_solver::kRing), group = slot / gy_solver::kGroup;
+    if (slot % gy_solver::kGroup == 0 && h->ring_busy[group]) CK(h, cudaEventSynchronize(h->ring_ev[group]));
+    h->epoch = h->epoch == 0x7fffffff ? 1 : h->epoch + 1;
+    h->h_ring[slot] = make_scalars(h, step);
     if (h->opt.use_graph && !timing) {
         StepGraph *gr = nullptr;
         for (auto &c : h->graphs)
@@ -1152,6 +1154,11 @@ static gy_status enqueue_step(gy_solver *h, double t, int step)
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(h, GY_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
     // host bookkeeping
+    h->ring_pos++;
+    if (slot % gy_solver::kGroup == gy_solver::kGroup - 1) {
+        CK(h, cudaEventRecord(h->ring_ev[group], s));
+        h->ring_busy[group] = true;
+    }
     if (v.sort) {
         h->sk = v.sk;
         h->since_sort = 0;
@@ -1351,8 +1358,7 @@ gy_status gy_get_stats(gy_solver *h, gy_stats *out)
     double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const double *part = h->h_rb->part;
     const int *flags = h->h_rb->flags;
-    CK(h, cudaMemcpyAsync(h->h_rb->part, h->d_stats, sizeof(h->h_rb->part), cudaMemcpyDeviceToHost, h->stream));
-    CK(h, cudaMemcpyAsync(h->h_rb->flags, h->d_status, sizeof(h->h_rb->flags), cudaMemcpyDeviceToHost, h->stream));
+    CK(h, cudaMemcpyAsync(h->h_rb, h->d_stats, sizeof(*h->h_rb), cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
     for (int q = 0; q < STATS_SLOTS; q++)
         for (int k = 1; k < 8; k++) v[k] += part[q * 8 + k];

@@ -79,13 +79,14 @@ __device__ __forceinline__ Sums cta_scan(Sums v, Sums *wsum, Sums *total)
 // CTAS > 1: each CTA of the cluster takes a contiguous share of the blocks; it sums the share,
 // learns the shares before its own through distributed shared memory, and scans it.  first_new is
 // written, the entering counts are cleared for the next G2P and the movers
-// grouped by their new block.  clear0 to clear3 (may be null): counters of the caller zeroed on
+// grouped by their new block; the step's
+// scalars are taken.  clear0 to clear3 (may be null): counters of the caller zeroed on
 // the way.
 // It is all latency: a grid of 125 blocks took 10 us in eight CTAs, of which the three cluster
 // barriers and the exchange were half; one CTA takes 3.4 us, and is the faster one up to BS_ONE
 // blocks (two tiles of BS_TILE).  54,000 blocks take 16 us in the cluster.
 template <int CTAS>
-__device__ __forceinline__ void blocks_scan(const BlockSort &b, int *first_new, int piece, int *nseg, int *clear0,
+__device__ __forceinline__ void blocks_scan(const BlockSort &b, const ScalarRing &ring, int *first_new, int piece, int *nseg, int *clear0,
                                             int *clear1, int *clear2, int *clear3)
 {
     __shared__ Sums wsum[BS_WARPS];
@@ -93,6 +94,7 @@ __device__ __forceinline__ void blocks_scan(const BlockSort &b, int *first_new, 
     pdl_prologue();
     const int tid = threadIdx.x, rank = CTAS > 1 ? (int)blockIdx.x : 0;
     const int nmov = *b.mov_n;
+    if (rank == 0 && tid >= BS_THREADS - 32) take_scalars(ring);
     if (rank == 0 && tid == 0) {
         if (clear0) *clear0 = 0;
         if (clear1) *clear1 = 0;
@@ -173,14 +175,16 @@ __device__ __forceinline__ void blocks_scan(const BlockSort &b, int *first_new, 
     }
 }
 __global__ void __cluster_dims__(BS_CTAS, 1, 1) __launch_bounds__(BS_THREADS)
-    k_blocks_scan(BlockSort b, int *first_new, int piece, int *nseg, int *clear0, int *clear1, int *clear2, int *clear3)
+    k_blocks_scan(BlockSort b, ScalarRing ring, int *first_new, int piece, int *nseg, int *clear0, int *clear1, int *clear2,
+                  int *clear3)
 {
-    blocks_scan<BS_CTAS>(b, first_new, piece, nseg, clear0, clear1, clear2, clear3);
+    blocks_scan<BS_CTAS>(b, ring, first_new, piece, nseg, clear0, clear1, clear2, clear3);
 }
 __global__ void __launch_bounds__(BS_THREADS)
-    k_blocks_scan_one(BlockSort b, int *first_new, int piece, int *nseg, int *clear0, int *clear1, int *clear2, int *clear3)
+    k_blocks_scan_one(BlockSort b, ScalarRing ring, int *first_new, int piece, int *nseg, int *clear0, int *clear1, int *clear2,
+                  int *clear3)
 {
-    blocks_scan<1>(b, first_new, piece, nseg, clear0, clear1, clear2, clear3);
+    blocks_scan<1>(b, ring, first_new, piece, nseg, clear0, clear1, clear2, clear3);
 }
 
 // key: the particles' keys in the old order.  A block's members are numbered movers from lower
@@ -392,13 +396,23 @@ void launch_blocks_count(const BlockSort &b, const int *skey, long long n, cudaS
     note_launch(1);
 }
 
-void launch_blocks_scan(const BlockSort &b, int which, int piece, int *nseg, cudaStream_t s, int *clear0, int *clear1,
-                        int *clear2, int *clear3)
+__global__ void k_take_scalars(ScalarRing ring) { take_scalars(ring); }
+
+void launch_take_scalars(const ScalarRing &ring, cudaStream_t s)
+{
+    k_take_scalars<<<1, 32, 0, s>>>(ring);
+    note_launch(1);
+}
+
+void launch_blocks_scan(const BlockSort &b, const ScalarRing &ring, int which, int piece, int *nseg, cudaStream_t s,
+                        int *clear0, int *clear1, int *clear2, int *clear3)
 {
     if (b.nblk <= BS_ONE)
-        launch_pdl(k_blocks_scan_one, 1, BS_THREADS, s, b, b.first[which], piece, nseg, clear0, clear1, clear2, clear3);
+        launch_pdl(k_blocks_scan_one, 1, BS_THREADS, s, b, ring, b.first[which], piece, nseg, clear0, clear1, clear2,
+                   clear3);
     else
-        launch_pdl(k_blocks_scan, BS_CTAS, BS_THREADS, s, b, b.first[which], piece, nseg, clear0, clear1, clear2, clear3);
+        launch_pdl(k_blocks_scan, BS_CTAS, BS_THREADS, s, b, ring, b.first[which], piece, nseg, clear0, clear1, clear2,
+                   clear3);
     note_launch(1);
 }
 

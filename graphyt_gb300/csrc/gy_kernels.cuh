@@ -84,6 +84,28 @@ struct BlockSort {
     int nblk;
 };
 
+// The steps' scalars in pinned host memory, one slot per step in turn.  The first kernel of a step
+// takes the next slot into `sc`, where the others read it: a copy
+// ahead of the step's kernels cost a small step 3 of its 33 us.
+struct ScalarRing {
+    static constexpr int SLOTS = 32;
+    const StepScalars *slots;
+    int *taken;              // the slot the next step takes
+    StepScalars *sc;
+};
+#ifdef __CUDACC__
+// by one warp
+__device__ __forceinline__ void take_scalars(const ScalarRing &r)
+{
+    const int lane = threadIdx.x & 31, t = *r.taken;
+    static_assert(sizeof(StepScalars) <= 32 * sizeof(int), "a lane per word");
+    if (lane < (int)(sizeof(StepScalars) / sizeof(int)))
+        reinterpret_cast<int *>(r.sc)[lane] = __ldcv(reinterpret_cast<const int *>(r.slots + t) + lane);
+    __syncwarp();
+    if (lane == 0) *r.taken = (t + 1) % ScalarRing::SLOTS;
+}
+#endif
+
 struct StepArgs {
     GridGeom g;
     const StepScalars *sc;   // per-step scalars in device memory (one small copy per step)
@@ -220,8 +242,9 @@ void resort_keys(const int *key, const int *prev_skey, int *skey_out, int *perm_
 size_t block_sort_ints(long long nblk, long long cap);
 void block_sort_bind(BlockSort &b, int *mem, long long nblk, long long cap);
 void launch_blocks_count(const BlockSort &b, const int *skey, long long n, cudaStream_t s);
-void launch_blocks_scan(const BlockSort &b, int which, int piece, int *nseg, cudaStream_t s, int *clear0 = nullptr,
-                        int *clear1 = nullptr, int *clear2 = nullptr, int *clear3 = nullptr);
+void launch_blocks_scan(const BlockSort &b, const ScalarRing &ring, int which, int piece, int *nseg, cudaStream_t s,
+                        int *clear0 = nullptr, int *clear1 = nullptr, int *clear2 = nullptr, int *clear3 = nullptr);
+void launch_take_scalars(const ScalarRing &ring, cudaStream_t s);
 // key null: another sort has made the order, only the segments are written
 void launch_blocks_place(const BlockSort &b, const int *key, int which, int piece, int *seg_start, int *seg_len,
                          int *skey_out, int *perm_out, long long n, cudaStream_t s);
