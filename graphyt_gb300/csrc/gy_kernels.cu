@@ -2338,6 +2338,29 @@ __device__ __forceinline__ void g2p_node_sums(const float4 *TV, const float2 *TA
     th[0] = gtx; th[1] = gty; th[2] = gtz; th[3] = trate;
 }
 
+// The loads of the particle a G2P thread takes next, issued ahead of their use: first its key and
+// slot, then its offsets (registers) and the rest of its state (the thread's own column of stage,
+// whose values the thread has taken out by then).
+struct G2PNext {
+    int key = -1, j = 0;  // key -1: none
+    float o[3];
+    __device__ __forceinline__ void slot(const int *skey, const int *perm, long long i, long long end)
+    {
+        key = i < end ? skey[i] : -1;
+        j = i < end ? perm[i] : 0;
+    }
+    template <int NST, int NT>
+    __device__ __forceinline__ void fields(const PView &src, float (*stage)[NT])
+    {
+        if (key < 0) return;
+#pragma unroll
+        for (int k = 0; k < 3; k++) o[k] = src.f(PF_OX + k, j);
+#pragma unroll
+        for (int f = 0; f < NST; f++) cp_async4(&stage[f][threadIdx.x], &src.f(g2p_stage_field(f), j));
+        cp_async_commit();
+    }
+};
+
 // Single-body G2P + update through a shared-memory node tile.  A CTA owns one segment (the
 // particles of one 4x4x4 cell block): it loads the block's 6x6x6 solved node tile once, with
 // massless nodes zeroed (they are skipped, Extrapolation.cpp:301-303), then runs one thread
@@ -2346,7 +2369,15 @@ __device__ __forceinline__ void g2p_node_sums(const float4 *TV, const float2 *TA
 // THERMAL adds the heat conduction terms (Extrapolation.cpp:132-134, 358-362 and
 // TimeIntegration.cpp:49-50): the node (T, rate) tile, the particle's temperature gradient and
 // rate summed with the same weights, and its temperature update, in therm by insertion index.
-template <bool HAS_DP, bool THERMAL>
+// What bounds it is latency: 62 % of the stalls wait for global loads, half the issue slots are
+// taken, DRAM at 39 % (2.4 million particles; a copy of the same bytes would take half as long).
+// AHEAD: the loads of a segment's first particles travel with those of its node tile, and a
+// thread's next particle loads while the current one is updated: G2P 133.0 -> 124.6 us at 2.4
+// million particles, 47.7 -> 44.7 at 730,000.  Loading ahead across segments as well gave 129.9,
+// for what is loaded early then stays in the way of the other CTAs' tiles.  With the wider state of
+// plasticity and damage the five more registers spill (24.6 -> 26.0 us at 184,000 particles), and
+// with heat conduction it gained nothing (a 2D plate's step 30.3 -> 31.0), so both load at use.
+template <bool HAS_DP, bool THERMAL, bool AHEAD>
 __global__ void __launch_bounds__(GY_G2P_THREADS, THERMAL ? GY_G2P_MINB_TH : GY_G2P_MINB)
     k_g2p_tiled(PView src, PView dst, const int *perm, const int *skey, long long n, Segs sg, int sorted, NodeBufs nb, StepArgs a, int check_finite, float4 *therm,
                 const float2 *tnode)
@@ -2364,9 +2395,11 @@ __global__ void __launch_bounds__(GY_G2P_THREADS, THERMAL ? GY_G2P_MINB_TH : GY_
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < NSTAT; k++) s_st[k][tid] = 0.f;  // each thread's own column
+    G2PNext nx;
     for (int sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
         const long long start = sg.start[sgi], end = sg.len ? start + sg.len[sgi] : n;
         const int blk = seg_block(skey, start);
+        if (AHEAD) nx.slot(skey, perm, start + tid, end);  // travels with the tile
         int bx, by, bz;
         decode_block(blk, g, bx, by, bz);
         const int tox = bx * CB, toy = by * CB, toz = g.is3d ? bz * CB : 0;
@@ -2388,6 +2421,7 @@ __global__ void __launch_bounds__(GY_G2P_THREADS, THERMAL ? GY_G2P_MINB_TH : GY_
                 if (THERMAL) TNr[h] = __ldg(&tnode[nd]);
             }
         }
+        if (AHEAD) nx.fields<NST>(src, stage);
         __syncthreads();  // the previous segment's particles are done with the tile
 #pragma unroll
         for (int h = 0; h < TILE_ITERS; h++) {
@@ -2403,7 +2437,15 @@ __global__ void __launch_bounds__(GY_G2P_THREADS, THERMAL ? GY_G2P_MINB_TH : GY_
             int cnt, key = 0;
             long long j = 0;
             const long long i = base + tid;
-            if (sorted) {
+            float o[3];
+            if (AHEAD) {
+                cnt = (int)min((long long)blockDim.x, end - base);
+                if (base == start) __syncthreads();  // publishes the tile
+                key = nx.key;
+#pragma unroll
+                for (int k = 0; k < 3; k++) o[k] = nx.o[k];
+                nx.slot(skey, perm, i + blockDim.x, end);
+            } else if (sorted) {
                 // the particle's key and slot are loaded together; the barrier also publishes
                 // the tile.  skey[i] is the key of particle perm[i].
                 const bool inr = i < end;
@@ -2424,12 +2466,17 @@ __global__ void __launch_bounds__(GY_G2P_THREADS, THERMAL ? GY_G2P_MINB_TH : GY_
             if (tid < cnt) {
                 PState st;
                 st.key = key;
+                if (AHEAD) {
 #pragma unroll
-                for (int k = 0; k < 3; k++) st.o[k] = src.f(PF_OX + k, j);
-                // the rest of the state travels to shared memory during the G2P sums
+                    for (int k = 0; k < 3; k++) st.o[k] = o[k];
+                } else {
 #pragma unroll
-                for (int f = 0; f < NST; f++) cp_async4(&stage[f][tid], &src.f(g2p_stage_field(f), j));
-                cp_async_commit();
+                    for (int k = 0; k < 3; k++) st.o[k] = src.f(PF_OX + k, j);
+                    // the rest of the state travels to shared memory during the G2P sums
+#pragma unroll
+                    for (int f = 0; f < NST; f++) cp_async4(&stage[f][tid], &src.f(g2p_stage_field(f), j));
+                    cp_async_commit();
+                }
                 float acc[3], vg[3], L[3][3], thg[4];
                 g2p_node_sums<THERMAL>(TV, TA, TN, st.o, st.key, g, acc, vg, L, thg);
                 cp_async_wait_all();
@@ -2457,11 +2504,14 @@ __global__ void __launch_bounds__(GY_G2P_THREADS, THERMAL ? GY_G2P_MINB_TH : GY_
                     st.dmg = 0.f;
                     st.smax = 0.f;
                 }
+                if (AHEAD) nx.fields<NST>(src, stage);
                 float4 th = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (THERMAL) th = therm[st.pid];  // loads while the update runs
-                int c0[3];
-                decode_key(st.key, g, c0[0], c0[1], c0[2]);
-                if (!g.is3d) c0[2] = 0;
+                int c0[3] = {tox + (key & 3), toy + ((key >> 2) & 3), g.is3d ? toz + ((key >> 4) & 3) : 0};
+                if (!AHEAD) {  // where registers are short, the corner is not kept
+                    decode_key(st.key, g, c0[0], c0[1], c0[2]);
+                    if (!g.is3d) c0[2] = 0;
+                }
                 update_after_g2p<HAS_DP>(st, c0, acc, vg, L, a, check_finite != 0, i);
                 store_state<HAS_DP>(dst, i, st);
                 if (st.key != key && (a.mover_mask || a.blk_cnt)) flag_mover(a, i, key, st.key);
@@ -2682,8 +2732,8 @@ __global__ void __launch_bounds__(GY_G2PM_THREADS, GY_G2PM_MINB) k_g2p_multi_til
 int g2p_blocks_per_sm(bool has_dp)
 {
     int b = 0;
-    if (has_dp) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_g2p_tiled<true, false>, GY_G2P_THREADS, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_g2p_tiled<false, false>, GY_G2P_THREADS, 0);
+    if (has_dp) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_g2p_tiled<true, false, false>, GY_G2P_THREADS, 0);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_g2p_tiled<false, false, false>, GY_G2P_THREADS, 0);
     return b > 0 ? b : 1;
 }
 
@@ -2726,21 +2776,34 @@ void launch_g2p_update(const PView &src, const PView &dst, const int *perm, cons
                 int dev = 0, sms = 1, b = 0;
                 cudaGetDevice(&dev);
                 cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-                if (has_dp) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_g2p_tiled<true, true>, GY_G2P_THREADS, 0);
-                else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_g2p_tiled<false, true>, GY_G2P_THREADS, 0);
+                if (has_dp) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_g2p_tiled<true, true, false>, GY_G2P_THREADS, 0);
+                else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_g2p_tiled<false, true, false>, GY_G2P_THREADS, 0);
                 tgrid[has_dp] = sms * std::max(b, 1);
             }
             if (has_dp)
-                launch_step(k_g2p_tiled<true, true>, seg_grid(tgrid[1], sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n,
+                launch_step(k_g2p_tiled<true, true, false>, seg_grid(tgrid[1], sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n,
                            sg, srt, nb, a, cf, therm, tnode);
             else
-                launch_step(k_g2p_tiled<false, true>, seg_grid(tgrid[0], sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n,
+                launch_step(k_g2p_tiled<false, true, false>, seg_grid(tgrid[0], sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n,
                            sg, srt, nb, a, cf, therm, tnode);
         } else if (has_dp) {
-            launch_step(k_g2p_tiled<true, false>, seg_grid(g2p_grid, sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n, sg,
+            launch_step(k_g2p_tiled<true, false, false>, seg_grid(g2p_grid, sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n, sg,
                        srt, nb, a, cf, (float4 *)nullptr, (const float2 *)nullptr);
+        } else if (sg.len && perm && sg.most > g2p_grid) {
+            // where the chip holds all segments at once there is nothing to load ahead of (the 8k
+            // cube's step 27.1 us, loading ahead 27.5)
+            static int agrid = 0;  // persistent grid of the variant
+            if (agrid == 0) {
+                int dev = 0, sms = 1, b = 0;
+                cudaGetDevice(&dev);
+                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_g2p_tiled<false, false, true>, GY_G2P_THREADS, 0);
+                agrid = sms * std::max(b, 1);
+            }
+            launch_step(k_g2p_tiled<false, false, true>, seg_grid(agrid, sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n,
+                       sg, srt, nb, a, cf, (float4 *)nullptr, (const float2 *)nullptr);
         } else {
-            launch_step(k_g2p_tiled<false, false>, seg_grid(g2p_grid, sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n, sg,
+            launch_step(k_g2p_tiled<false, false, false>, seg_grid(g2p_grid, sg.most), GY_G2P_THREADS, s, src, dst, perm, skey, n, sg,
                        srt, nb, a, cf, (float4 *)nullptr, (const float2 *)nullptr);
         }
     }
