@@ -162,9 +162,14 @@ static constexpr long long BLOCK_SORT_MAX = 1 << 20;
 // 256 / whole blocks: 43 / 46 / 57 / 76 us at 8,000 particles, 67 / 67 / 81 / 108 at 86,000,
 // 90 / 85 / 99 / 127 at 184,000, 164 / 154 / 169 / 157 at 730,000, 394 / 365 / 395 / 375 at 2.4
 // million.
-static int segment_piece(long long n)
+// A remainder that would not fill a warp goes with the piece before it where there are many more
+// segments than resident warps (a step of 2.4 million particles 341 -> 329 us, of 730,000 133.7 ->
+// 133.1); with fewer the longer pieces make the tail longer (184,000 particles 63.2 -> 65.7 us),
+// and with several bodies, whose pieces are one chunk of a CTA, they take another pass (24 impacts
+// of 1.1 million 316 -> 319).
+static Pieces segment_pieces(long long n, bool multi)
 {
-    return n >= 100000 ? 128 : 64;
+    return {n >= 100000 ? 128 : 64, n >= 500000 && !multi ? 32 : 0};
 }
 
 namespace {
@@ -1037,13 +1042,13 @@ static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
     if (v.blocks || v.sort == 3) {
         // a sort from scratch counts the blocks; after it G2P keeps the counts
         if (v.sort != 3) launch_blocks_count(h->bs, skey, h->n, s);
-        const int piece = segment_piece(h->n);
+        const Pieces piece = segment_pieces(h->n, h->multi);
         launch_blocks_scan(h->bs, ring, v.fb, piece, nseg, s, h->nb.active_n, h->nb.active_count, h->d_nseg + (v.cur ^ 1),
                            ndefer);
         launch_blocks_place(h->bs, v.sort == 3 ? key : nullptr, v.fb, piece, h->d_seg, h->d_seglen, h->skey_buf[v.sk],
                             h->d_perm, h->n, s);
         sg.len = h->d_seglen;
-        sg.most = h->n / segment_piece(h->n) + std::min<long long>(h->bs.nblk, h->n);  // full pieces and remainders
+        sg.most = h->n / piece.len + std::min<long long>(h->bs.nblk, h->n);  // full pieces and remainders
     } else {
         // the segment count alternates between two counters by slab parity: this step's block
         // heads fill one and zero the other for the next step, and zero this step's active

@@ -8,12 +8,13 @@
 // then takes two launches:
 //   k_blocks_scan   one cluster: the blocks' first positions (a prefix sum of the counts), the
 //                   non-empty blocks, the place of each one's segments among those the particle
-//                   kernels take (a block's particles, in pieces of at most `piece`), and the
-//                   movers grouped by their new block;
-//   k_blocks_place  a CTA per non-empty block: its segments, the permutation and the sorted keys.  A block that
-//                   nothing entered, left or changed cell in is copied; the others are sorted by
-//                   (cell, old slot), a stable counting sort over their 64 cells of the movers from
-//                   lower slots, the old range and the movers from higher slots, in this order.
+//                   kernels take (a block's particles in pieces), and the movers grouped by their
+//                   new block;
+//   k_blocks_place  a CTA per non-empty block: its segments, the permutation and the sorted keys.
+//                   A block that nothing entered, left or changed cell in is copied; the others
+//                   are sorted by (cell, old slot), a stable counting sort over their 64 cells of
+//                   the movers from lower slots, the old range and the movers from higher slots,
+//                   in this order.
 // The result is the permutation of a stable sort of all keys.  It replaced ten launches (a merge
 // of all movers with all stayers through particle-wide prefix sums: gy_resort.cu, which still
 // serves sorts that several steps of movement precede), whose launch latencies were most of the
@@ -40,9 +41,15 @@ struct Sums {
     int n, in, seg, ne;
 };
 __device__ __forceinline__ Sums operator+(Sums a, Sums b) { return {a.n + b.n, a.in + b.in, a.seg + b.seg, a.ne + b.ne}; }
-__device__ __forceinline__ Sums block_sums(int n, int in, int piece)
+// the segments a block's n particles are taken in
+__device__ __forceinline__ int block_pieces(int n, Pieces piece)
 {
-    return {n, in, (n + piece - 1) / piece, n > 0 ? 1 : 0};
+    return n <= piece.len ? (n > 0 ? 1 : 0) : (n - piece.merge + piece.len - 1) / piece.len;
+}
+
+__device__ __forceinline__ Sums block_sums(int n, int in, Pieces piece)
+{
+    return {n, in, block_pieces(n, piece), n > 0 ? 1 : 0};
 }
 __device__ __forceinline__ Sums shfl_up(Sums a, int d)
 {
@@ -86,7 +93,7 @@ __device__ __forceinline__ Sums cta_scan(Sums v, Sums *wsum, Sums *total)
 // barriers and the exchange were half; one CTA takes 3.4 us, and is the faster one up to BS_ONE
 // blocks (two tiles of BS_TILE).  54,000 blocks take 16 us in the cluster.
 template <int CTAS>
-__device__ __forceinline__ void blocks_scan(const BlockSort &b, const ScalarRing &ring, int *first_new, int piece, int *nseg, int *clear0,
+__device__ __forceinline__ void blocks_scan(const BlockSort &b, const ScalarRing &ring, int *first_new, Pieces piece, int *nseg, int *clear0,
                                             int *clear1, int *clear2, int *clear3)
 {
     __shared__ Sums wsum[BS_WARPS];
@@ -175,13 +182,13 @@ __device__ __forceinline__ void blocks_scan(const BlockSort &b, const ScalarRing
     }
 }
 __global__ void __cluster_dims__(BS_CTAS, 1, 1) __launch_bounds__(BS_THREADS)
-    k_blocks_scan(BlockSort b, ScalarRing ring, int *first_new, int piece, int *nseg, int *clear0, int *clear1, int *clear2,
+    k_blocks_scan(BlockSort b, ScalarRing ring, int *first_new, Pieces piece, int *nseg, int *clear0, int *clear1, int *clear2,
                   int *clear3)
 {
     blocks_scan<BS_CTAS>(b, ring, first_new, piece, nseg, clear0, clear1, clear2, clear3);
 }
 __global__ void __launch_bounds__(BS_THREADS)
-    k_blocks_scan_one(BlockSort b, ScalarRing ring, int *first_new, int piece, int *nseg, int *clear0, int *clear1, int *clear2,
+    k_blocks_scan_one(BlockSort b, ScalarRing ring, int *first_new, Pieces piece, int *nseg, int *clear0, int *clear1, int *clear2,
                   int *clear3)
 {
     blocks_scan<1>(b, ring, first_new, piece, nseg, clear0, clear1, clear2, clear3);
@@ -198,18 +205,19 @@ __global__ void __launch_bounds__(BS_THREADS)
 constexpr int BP_PER = 4;
 constexpr int BP_ROUND = BP_THREADS * BP_PER;
 // the segments of the block at `s` in the list (a few: written by the CTA's first threads)
-__device__ __forceinline__ void put_segments(const BlockSort &b, int s, int nf, int nc, int piece, int *seg_start,
+__device__ __forceinline__ void put_segments(const BlockSort &b, int s, int nf, int nc, Pieces piece, int *seg_start,
                                              int *seg_len)
 {
     const int at = b.seg_at[s];
-    for (int k = threadIdx.x; (long long)k * piece < nc; k += blockDim.x) {
-        seg_start[at + k] = nf + k * piece;
-        seg_len[at + k] = min(piece, nc - k * piece);
+    const int np = block_pieces(nc, piece);
+    for (int k = threadIdx.x; k < np; k += blockDim.x) {
+        seg_start[at + k] = nf + k * piece.len;
+        seg_len[at + k] = k < np - 1 ? piece.len : nc - k * piece.len;
     }
 }
 
 // the segments alone, of an order that another sort made
-__global__ void __launch_bounds__(BP_THREADS) k_blocks_segments(BlockSort b, const int *first_new, int piece,
+__global__ void __launch_bounds__(BP_THREADS) k_blocks_segments(BlockSort b, const int *first_new, Pieces piece,
                                                                 int *seg_start, int *seg_len)
 {
     for (int s = blockIdx.x; s < *b.list_n; s += gridDim.x) {
@@ -219,7 +227,7 @@ __global__ void __launch_bounds__(BP_THREADS) k_blocks_segments(BlockSort b, con
 }
 
 __global__ void __launch_bounds__(BP_THREADS, 12) k_blocks_place(BlockSort b, const int *key, const int *first_old,
-                                                             const int *first_new, int piece, int *seg_start, int *seg_len,
+                                                             const int *first_new, Pieces piece, int *seg_start, int *seg_len,
                                                              int *skey_out, int *perm_out)
 {
     __shared__ int next[64];            // next position of each cell, in the rounds after the first
@@ -404,7 +412,7 @@ void launch_take_scalars(const ScalarRing &ring, cudaStream_t s)
     note_launch(1);
 }
 
-void launch_blocks_scan(const BlockSort &b, const ScalarRing &ring, int which, int piece, int *nseg, cudaStream_t s,
+void launch_blocks_scan(const BlockSort &b, const ScalarRing &ring, int which, Pieces piece, int *nseg, cudaStream_t s,
                         int *clear0, int *clear1, int *clear2, int *clear3)
 {
     if (b.nblk <= BS_ONE)
@@ -416,7 +424,7 @@ void launch_blocks_scan(const BlockSort &b, const ScalarRing &ring, int which, i
     note_launch(1);
 }
 
-void launch_blocks_place(const BlockSort &b, const int *key, int which, int piece, int *seg_start, int *seg_len,
+void launch_blocks_place(const BlockSort &b, const int *key, int which, Pieces piece, int *seg_start, int *seg_len,
                          int *skey_out, int *perm_out, long long n, cudaStream_t s)
 {
     static int sms = 0;

@@ -69,6 +69,12 @@ struct Segs {
     long long most;   // there are no more of them than this (0: not known)
 };
 
+// How a cell block's particles are cut into segments: pieces of len, and a remainder of up to merge
+// goes with the last of them.
+struct Pieces {
+    int len, merge;
+};
+
 // Cell-block bookkeeping of the block merge sort (gy_blocks.cu); zeroed once at allocation.
 struct BlockSort {
     int *cnt;             // particles per cell block by their current key, kept by G2P
@@ -242,11 +248,11 @@ void resort_keys(const int *key, const int *prev_skey, int *skey_out, int *perm_
 size_t block_sort_ints(long long nblk, long long cap);
 void block_sort_bind(BlockSort &b, int *mem, long long nblk, long long cap);
 void launch_blocks_count(const BlockSort &b, const int *skey, long long n, cudaStream_t s);
-void launch_blocks_scan(const BlockSort &b, const ScalarRing &ring, int which, int piece, int *nseg, cudaStream_t s,
+void launch_blocks_scan(const BlockSort &b, const ScalarRing &ring, int which, Pieces piece, int *nseg, cudaStream_t s,
                         int *clear0 = nullptr, int *clear1 = nullptr, int *clear2 = nullptr, int *clear3 = nullptr);
 void launch_take_scalars(const ScalarRing &ring, cudaStream_t s);
 // key null: another sort has made the order, only the segments are written
-void launch_blocks_place(const BlockSort &b, const int *key, int which, int piece, int *seg_start, int *seg_len,
+void launch_blocks_place(const BlockSort &b, const int *key, int which, Pieces piece, int *seg_start, int *seg_len,
                          int *skey_out, int *perm_out, long long n, cudaStream_t s);
 // particle fields in insertion order and FP64 (gy_export.cu)
 struct ExportArgs {

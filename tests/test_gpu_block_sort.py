@@ -114,3 +114,22 @@ def test_particle_update_does_not_depend_on_how_many_segments_there_may_be(gpu_l
     for a, b, tol in zip(*out, (2e-5 * sc.dt, 2e-5, 3 * 2e-5)):
         assert np.isfinite(a).all() and np.ptp(a) > 0
         assert np.abs(a - b).max() <= tol * vmax
+
+
+def test_remainders_taken_with_the_last_piece(gpu_lib):
+    """512,000 particles, whose blocks' remainders of up to a warp go with the last piece, against
+    full_sort, which cuts no pieces; tolerances as above."""
+    from graphyt_gb300 import graphyt
+    out = []
+    for options in (None, dict(full_sort=1)):
+        sc = _fast_block(80, 0.5)
+        sc.L = [4.0, 4.0, 4.0]
+        sc.dt = 0.2 * sc.cellsize
+        s = graphyt.from_scene(sc, options=options)
+        s.iterate_GPU_steps(3)
+        out.append([s._get_particles(f) for f in ("pos", "vel", "stress")])
+        s.close()
+    vmax = np.abs(sc.vel).max()
+    for a, b, tol in zip(*out, (2e-5 * sc.dt, 2e-5, 3 * 2e-5)):
+        assert np.isfinite(a).all() and np.ptp(a) > 0
+        assert np.abs(a - b).max() <= tol * vmax
