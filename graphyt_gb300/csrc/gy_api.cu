@@ -161,7 +161,9 @@ static constexpr long long BLOCK_SORT_MAX = 1 << 20;
 // one, at the price of a node tile loaded and flushed per piece.  Step by piece length, 64 / 128 /
 // 256 / whole blocks: 43 / 46 / 57 / 76 us at 8,000 particles, 67 / 67 / 81 / 108 at 86,000,
 // 90 / 85 / 99 / 127 at 184,000, 164 / 154 / 169 / 157 at 730,000, 394 / 365 / 395 / 375 at 2.4
-// million.
+// million; -- / 636 / 622 / 603 at 5.0 million, -- / 1431 / 1420 / 1341 at 12.0, where even whole
+// blocks are several rounds of the resident warps, and with bodies -- / 1874 / 1647 / 1541 at 10.2
+// (a disc), -- / 2954 / 2865 / 2693 at 13.0 (256 impacts).
 // A remainder that would not fill a warp goes with the piece before it where there are many more
 // segments than resident warps (a step of 2.4 million particles 341 -> 329 us, of 730,000 133.7 ->
 // 133.1); with fewer the longer pieces make the tail longer (184,000 particles 63.2 -> 65.7 us),
@@ -169,8 +171,16 @@ static constexpr long long BLOCK_SORT_MAX = 1 << 20;
 // of 1.1 million 316 -> 319).
 static Pieces segment_pieces(long long n, bool multi)
 {
-    return {n >= 100000 ? 128 : 64, n >= 500000 && !multi ? 32 : 0};
+    if (n >= 4000000) return {10, 0};  // 1024: a full block of eight particles per cell holds 512
+    return {n >= 100000 ? 7 : 6, n >= 500000 && !multi ? 32 : 0};
 }
+
+// Particles from which the multi-body G2P takes whole cell blocks: its tile holds two bodies' node
+// fields, dear to load per piece, and it runs fewer and larger CTAs than P2G does warps.  G2P with
+// pieces / whole blocks: disc 25.0 / 27.0 us at 165,000 particles, 41.7 / 39.5 at 335,000, 75.2 /
+// 65.1 at 664,000, 138 / 114 at 1.3 million; impacts 38.5 / 43.5 at 265,000, 58.0 / 60.1 at 426,000,
+// 132.8 / 130.9 at 1.1 million.
+static constexpr long long G2P_WHOLE_BLOCKS = 500000;
 
 namespace {
 
@@ -1048,7 +1058,7 @@ static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
         launch_blocks_place(h->bs, v.sort == 3 ? key : nullptr, v.fb, piece, h->d_seg, h->d_seglen, h->skey_buf[v.sk],
                             h->d_perm, h->n, s);
         sg.len = h->d_seglen;
-        sg.most = h->n / piece.len + std::min<long long>(h->bs.nblk, h->n);  // full pieces and remainders
+        sg.most = h->n / piece.len() + std::min<long long>(h->bs.nblk, h->n);  // full pieces and remainders
     } else {
         // the segment count alternates between two counters by slab parity: this step's block
         // heads fill one and zero the other for the next step, and zero this step's active
@@ -1068,7 +1078,7 @@ static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
     // (b) P2G
     // heat conduction: fused into the single-body P2G, a separate pass for body slots
     const bool fused_thermal = h->thermal && !h->multi;
-    // multi-body: the one-object segments take the plane-lane kernel unless normals are tracked
+    // multi-body: the one-object segments take the one-body kernel unless normals are tracked
     int *defer = ndefer ? h->d_seg + h->cap : nullptr;
     launch_p2g(src, perm, skey, h->n, sg, h->persist_grid, h->nb, a, s,
                fused_thermal ? h->d_therm : nullptr, fused_thermal ? h->d_tnode : nullptr, h->opt.p2g_lanes, defer,
@@ -1083,7 +1093,14 @@ static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
     // (d) G2P + particle BCs + update + constitutive + damage, written in sorted order, with
     // the conservation sums of the updated state (their partials zeroed by the fold)
     if (h->surr_on) cudaMemsetAsync(h->d_pend_n, 0, sizeof(unsigned int), s);
-    launch_g2p_update(src, dst, perm, skey, h->n, sg, h->g2p_grid, h->nb, a,
+    Segs gs = sg;
+    if (h->multi && sg.len && h->n >= G2P_WHOLE_BLOCKS) {
+        gs.blk = h->bs.list;
+        gs.first = h->bs.first[v.fb];
+        gs.n = h->bs.list_n;
+        gs.most = std::min<long long>(h->bs.nblk, h->n);
+    }
+    launch_g2p_update(src, dst, perm, skey, h->n, gs, h->g2p_grid, h->nb, a,
                       h->opt.track_normals != 0, h->opt.check_finite != 0, h->has_dp, s,
                       fused_thermal ? h->d_therm : nullptr, fused_thermal ? h->d_tnode : nullptr);
     if (h->surr_on)

@@ -44,7 +44,7 @@ __device__ __forceinline__ Sums operator+(Sums a, Sums b) { return {a.n + b.n, a
 // the segments a block's n particles are taken in
 __device__ __forceinline__ int block_pieces(int n, Pieces piece)
 {
-    return n <= piece.len ? (n > 0 ? 1 : 0) : (n - piece.merge + piece.len - 1) / piece.len;
+    return n <= piece.len() ? (n > 0 ? 1 : 0) : (n - piece.merge + piece.len() - 1) >> piece.shift;
 }
 
 __device__ __forceinline__ Sums block_sums(int n, int in, Pieces piece)
@@ -211,8 +211,8 @@ __device__ __forceinline__ void put_segments(const BlockSort &b, int s, int nf, 
     const int at = b.seg_at[s];
     const int np = block_pieces(nc, piece);
     for (int k = threadIdx.x; k < np; k += blockDim.x) {
-        seg_start[at + k] = nf + k * piece.len;
-        seg_len[at + k] = k < np - 1 ? piece.len : nc - k * piece.len;
+        seg_start[at + k] = nf + (k << piece.shift);
+        seg_len[at + k] = k < np - 1 ? piece.len() : nc - (k << piece.shift);
     }
 }
 

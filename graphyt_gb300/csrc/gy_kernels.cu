@@ -1,14 +1,14 @@
 // gy_kernels.cu -- the GB300 kernels of one explicit GIMP MPM step.
 //
 // Data flow of a step (single body, the fast path):
-//   sort      stable counting sort of the particle cell keys (gy_sort.cu) -> perm, plus the
-//             list of non-empty 4x4x4 cell blocks ("segments");
+//   sort      stable sort of the particle cell keys (gy_blocks.cu; gy_sort.cu at first) -> perm,
+//             plus the segments: pieces of the non-empty 4x4x4 cell blocks;
+//   P2G       one warp per segment: particles of a run of equal cell are summed in registers
+//             and added into the warp's own shared-memory node tile, flushed with vector
+//             reductions (Extrapolation.cpp:166-286); where several bodies meet a CTA per
+//             segment keeps the centre-of-mass and both body-slot fields in its tile (a lane
+//             per stencil node);
 //   fold      periodic node-layer fold of the accumulated P2G fields (Grid.cpp:310-795);
-//   P2G       one CTA per segment: particles of a run of equal cell are summed in registers
-//             (nine lanes per run, a lane per x column of three stencil nodes) into a
-//             shared-memory node tile, flushed with vector reductions (Extrapolation.cpp:
-//             166-286); multi-body problems keep the centre-of-mass and both body-slot
-//             fields in the tile (a lane per stencil node);
 //   solve     nodal momentum update + grid BCs over the active 4x4x4 node blocks only
 //             (Grid.cpp:9-245, 862-1094); it also clears the accumulators it read;
 //   G2P       one CTA per segment over a shared-memory tile of the solved nodes, a thread
@@ -2548,8 +2548,17 @@ __global__ void __launch_bounds__(GY_G2PM_THREADS, GY_G2PM_MINB) k_g2p_multi_til
 #pragma unroll
     for (int k = 0; k < NSTAT; k++) s_st[k][tid] = 0.f;  // each thread's own column
     for (int sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
-        const long long start = sg.start[sgi], end = sg.len ? start + sg.len[sgi] : n;
-        const int blk = seg_block(skey, start);
+        long long start, end;
+        int blk;
+        if (sg.blk) {
+            blk = sg.blk[sgi];
+            start = sg.first[blk];
+            end = sg.first[blk + 1];
+        } else {
+            start = sg.start[sgi];
+            end = sg.len ? start + sg.len[sgi] : n;
+            blk = seg_block(skey, start);
+        }
         int bx, by, bz;
         decode_block(blk, g, bx, by, bz);
         const int tox = bx * CB, toy = by * CB, toz = g.is3d ? bz * CB : 0;
@@ -2935,7 +2944,7 @@ __global__ void __launch_bounds__(64) k_body_assign(NodeBufs nb, GridGeom g, con
 
 // Per 4x4x4 cell block, the body of its 6x6x6 node tile when the tile has one (every node with
 // body pair (b, -1) or (-1, -1)): b, -1 for none, -2 for two or more; one warp per block.
-// P2G sends the one-object segments of such blocks to the plane-lane kernel.
+// P2G sends the one-object segments of such blocks to the one-body kernel.
 __global__ void __launch_bounds__(128) k_block_body(NodeBufs nb, GridGeom g)
 {
     const int lane = threadIdx.x & 31;

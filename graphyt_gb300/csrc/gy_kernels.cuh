@@ -67,12 +67,14 @@ struct Segs {
     const int *start, *len;
     const int *n;
     long long most;   // there are no more of them than this (0: not known)
+    const int *blk = nullptr, *first = nullptr;  // with blk: whole cell blocks instead, [first[b], first[b + 1])
 };
 
-// How a cell block's particles are cut into segments: pieces of len, and a remainder of up to merge
-// goes with the last of them.
+// How a cell block's particles are cut into segments: pieces of 2^shift, and a remainder of up to
+// merge goes with the last of them.
 struct Pieces {
-    int len, merge;
+    int shift, merge;
+    __host__ __device__ int len() const { return 1 << shift; }
 };
 
 // Cell-block bookkeeping of the block merge sort (gy_blocks.cu); zeroed once at allocation.
@@ -187,7 +189,7 @@ void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, c
                 int *ndefer = nullptr);
 void launch_fold(const NodeBufs &nb, const StepArgs &a, cudaStream_t s);
 void launch_block_body(const NodeBufs &nb, const GridGeom &g, cudaStream_t s);
-// want_list: fill active_list / active_n (zeroed by the caller's block heads)
+// want_list: fill active_list / active_n (zeroed earlier in the step)
 void launch_solve(const NodeBufs &nb, const StepArgs &a, bool keep_node_fields, bool want_list, cudaStream_t s);
 // therm / tnode non-null: the single-body kernel also runs the heat conduction G2P and the
 // temperature update (multi-body problems run launch_thermal_g2p instead)

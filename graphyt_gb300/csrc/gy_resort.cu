@@ -13,7 +13,8 @@
 //   * stayer r (r-th stayer in slot order) lands at r + (movers with g <= r).
 // A bucket holding more than RS_BUCKET_MAX movers (a flow far outside the time-step limit,
 // or keys that are not cells) sends all movers through a one-CTA stable radix sort instead.
-// In the step the movers come flagged: G2P sets a bit per slot whose key it changes (with a
+// It serves the sorts that several steps of movement precede, and grids of too many cell blocks for
+// the block merge (gy_blocks.cu).  In the step the movers come flagged: G2P sets a bit per slot whose key it changes (with a
 // count per 32 slots), and the stayer placement, their last reader, clears the bits.  The
 // result is the permutation the full stable radix sort produces, at a fraction of its traffic
 // when few particles move; the full sort runs whenever the previous order is not known

@@ -116,15 +116,23 @@ def test_particle_update_does_not_depend_on_how_many_segments_there_may_be(gpu_l
         assert np.abs(a - b).max() <= tol * vmax
 
 
-def test_remainders_taken_with_the_last_piece(gpu_lib):
-    """512,000 particles, whose blocks' remainders of up to a warp go with the last piece, against
-    full_sort, which cuts no pieces; tolerances as above."""
+@pytest.mark.parametrize("n_side, bodies", [(80, 1), (80, 2), (160, 1)])
+def test_large_problems_take_longer_segments(gpu_lib, n_side, bodies):
+    """512,000 particles of one body, whose blocks' remainders of up to a warp go with the last
+    piece, and of two bodies apart, whose particle update takes whole blocks; 4.1 million, whose P2G
+    takes whole blocks.  Against full_sort, which cuts no pieces; tolerances as above."""
     from graphyt_gb300 import graphyt
     out = []
     for options in (None, dict(full_sort=1)):
-        sc = _fast_block(80, 0.5)
-        sc.L = [4.0, 4.0, 4.0]
+        sc = _fast_block(n_side, 0.5)
+        sc.L = [6.0, 6.0, 6.0] if n_side == 160 else [4.0, 4.0, 4.0]
         sc.dt = 0.2 * sc.cellsize
+        if n_side == 160:
+            sc.vel[np.arange(sc.n) % 200 > 0] = 0.0  # (few, for the surface takes them one by one)
+        if bodies == 2:
+            far = sc.pos[:, 0] > sc.pos[:, 0].mean()
+            sc.obj[far] = 1
+            sc.pos[far, 0] += 0.75
         s = graphyt.from_scene(sc, options=options)
         s.iterate_GPU_steps(3)
         out.append([s._get_particles(f) for f in ("pos", "vel", "stress")])
