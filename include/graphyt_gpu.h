@@ -75,19 +75,21 @@ typedef struct gy_params {
 /* Tuning knobs that change speed, never results beyond summation order. */
 typedef struct gy_options {
     int sort_every;     /* reorder particle state by cell every n steps (>= 1) */
-    int full_sort;      /* 1: every sort is a full radix sort; 0: after the first, an incremental
-                           re-sort of the particles that changed cell (same permutation) */
+    int full_sort;      /* 1: every sort is a full radix sort; 0: after the first, a merge per
+                           cell block (or an incremental re-sort of the particles that
+                           changed cell, with sort_every > 1); same permutation */
     int use_graph;      /* 1 (default): each step replays a captured CUDA graph of its kernels,
                            the step's scalars reaching the device in one small copy; 0: the
                            kernels are launched one by one */
     int track_normals;  /* 1: keep per-particle contact normals (getNormalsArr) */
     int check_finite;   /* 1: flag NaN/Inf in particle state every step */
     int keep_node_fields; /* 1: keep centre-of-mass node velocity/force for node getters */
-    int p2g_lanes;      /* P2G (with or without heat conduction): lanes per run of equal cell, 3 (default:
-                           each lane sums a z-plane of nine stencil nodes) or 9 (each lane a
-                           column of three x nodes).  Multi-body problems without tracked
+    int p2g_lanes;      /* P2G (with or without heat conduction): 3 (default: a warp per piece of a cell
+                           block; in steps that do not sort or sort from scratch three lanes
+                           per run of equal cell, a z-plane of nine stencil nodes each) or 9
+                           (nine lanes per run, a column of three x nodes each).  Multi-body problems without tracked
                            normals: 3 sends the segments of one deformable object whose node
-                           tile holds that body only through the 3-lane kernel and the rest
+                           tile holds that body only through that kernel and the rest
                            through the body-slot kernel; 9 sends every segment through the
                            body-slot kernel.  Same sums, different speed */
 } gy_options;
@@ -215,7 +217,7 @@ gy_status gy_get_nodes(gy_solver *h, int field, double *out, int64_t count);
  * arrays; for testing the sort against a CPU stable sort. */
 gy_status gy_sort_keys(const int *keys, int64_t n, int *perm_out, int device);
 
-/* The incremental re-sort the step uses after its first sort (no counterpart in the
+/* The incremental re-sort that sorts after several steps of movement use (no counterpart in the
  * reference, whose Extrapolation.cpp:370-503 sorts from scratch).  prev_sorted[i] is the key
  * particle i had at the last sort, in that sort's order (non-decreasing); keys[i] is its key
  * now.  Result: the stable ascending order of keys, equal to gy_sort_keys(keys).  Host arrays;
