@@ -829,6 +829,12 @@ __global__ void __launch_bounds__(PP_THREADS, THERMAL ? GY_PP_MINB_TH : GY_PP_MI
 // instructions (190 with the weights formed by each lane from the offsets, and f_z unpacked).
 // Tile and staging take 15.8 KB, 14 warps per SM.
 //
+// What bounds it is the latency of loads and instructions at those 14 warps: 49 % of the issue
+// slots, 37 warp instructions per particle (26 with whole blocks as segments), DRAM at 13-25 % of
+// its peak.  P2G with the shared tile / this kernel: 21 / 11 us at 8,000 particles, 88 / 61 at
+// 730,000, 223 / 156 at 2.4 million, 850 / 625 at 12 million in a developed flow; disc of 1.3
+// million 170 / 117.
+//
 // MULTI, THERMAL: as in k_p2g_planes (a segment of several objects is left to `defer` before
 // anything of it is flushed).
 constexpr int PW_ROWS = 80;                          // particles of a chunk
@@ -1420,8 +1426,10 @@ void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, c
                 const float4 *therm, float2 *tnode, int lanes, int *defer, int *ndefer)
 {
     if (n == 0) return;
-    // a sorted step whose segments are known takes the warp kernel; 9 lanes ask for the column
-    // kernel (and on multi-body problems for the body-slot kernel throughout)
+    // a sorted step whose segments are known takes the warp kernel, which was the faster one at every
+    // size (above); the shared-tile kernels find a segment's end themselves and serve the other
+    // steps; 9 lanes ask for the column kernel (and on multi-body problems for the body-slot kernel
+    // throughout: 256 impacts 2.86 ms a step with 3, 3.02 with 9)
     const bool warps = lanes == 3 && perm && sg.len;
     if (warps && (!a.multi_body || (defer && ndefer))) {
         static int grid[3] = {0, 0, 0};  // resident warps of the three variants
