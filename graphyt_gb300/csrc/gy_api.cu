@@ -189,7 +189,7 @@ namespace {
 gy_status fail(gy_solver *h, gy_status code, const std::string &msg)
 {
     if (h) h->err = msg;
-    return code;
+    return code == GY_ERR_CUDA || code == GY_ERR_NOMEM ? cuda_failed(code) : code;
 }
 
 #define CK(h, call)                                                                        \
@@ -301,14 +301,14 @@ gy_status gy_create(const gy_grid_desc *grid, int device, gy_solver **out)
     if (device >= 0) {
         if (cudaSetDevice(device) != cudaSuccess) {
             delete s;
-            return GY_ERR_CUDA;
+            return cuda_failed(GY_ERR_CUDA);
         }
     } else {
         cudaGetDevice(&s->device);
     }
     if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) {
         delete s;
-        return GY_ERR_CUDA;
+        return cuda_failed(GY_ERR_CUDA);
     }
     for (int i = 0; i < 6; i++) cudaEventCreate(&s->ev[i]);
     for (int a = 0; a < 3; a++) s->L[a] = grid->L[a];
@@ -1561,7 +1561,7 @@ gy_status gy_sort_keys(const int *keys, int64_t n, int *perm_out, int device)
 {
     if (n < 0 || (n > 0 && (!keys || !perm_out))) return GY_ERR_ARG;
     if (n == 0) return GY_OK;
-    if (device >= 0 && cudaSetDevice(device) != cudaSuccess) return GY_ERR_CUDA;
+    if (device >= 0 && cudaSetDevice(device) != cudaSuccess) return cuda_failed(GY_ERR_CUDA);
     int maxk = 0;
     for (int64_t i = 0; i < n; i++) {
         if (keys[i] < 0) return GY_ERR_ARG;
@@ -1570,13 +1570,13 @@ gy_status gy_sort_keys(const int *keys, int64_t n, int *perm_out, int device)
     int bits = 1;
     while ((1LL << bits) <= maxk) bits++;
     cudaStream_t s;
-    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return GY_ERR_CUDA;
+    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return cuda_failed(GY_ERR_CUDA);
     int *d_in = nullptr, *d_perm = nullptr, *mem = nullptr;
     gy_status st = GY_OK;
     const long long nbk = (n + 2047) / 2048;
     if (cudaMalloc(&d_in, n * sizeof(int)) != cudaSuccess || cudaMalloc(&d_perm, n * sizeof(int)) != cudaSuccess ||
         cudaMalloc(&mem, sort_scratch_bytes(n) + 4096) != cudaSuccess) {
-        st = GY_ERR_NOMEM;
+        st = cuda_failed(GY_ERR_NOMEM);
     } else {
         SortScratch ws{};
         int *p = mem;
@@ -1591,7 +1591,7 @@ gy_status gy_sort_keys(const int *keys, int64_t n, int *perm_out, int device)
         cudaMemcpyAsync(d_in, keys, n * sizeof(int), cudaMemcpyHostToDevice, s);
         (void)sort_pairs(d_in, d_perm, n, bits, ws, s);
         cudaMemcpyAsync(perm_out, d_perm, n * sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (cudaStreamSynchronize(s) != cudaSuccess) st = GY_ERR_CUDA;
+        if (cudaStreamSynchronize(s) != cudaSuccess) st = cuda_failed(GY_ERR_CUDA);
     }
     if (d_in) cudaFree(d_in);
     if (d_perm) cudaFree(d_perm);
@@ -1615,14 +1615,14 @@ gy_status gy_resort_keys(const int *keys, const int *prev_sorted, int64_t n, int
     }
     int bits = 1;
     while ((1LL << bits) <= maxk) bits++;
-    if (device >= 0 && cudaSetDevice(device) != cudaSuccess) return GY_ERR_CUDA;
+    if (device >= 0 && cudaSetDevice(device) != cudaSuccess) return cuda_failed(GY_ERR_CUDA);
     cudaStream_t s;
-    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return GY_ERR_CUDA;
+    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return cuda_failed(GY_ERR_CUDA);
     int *mem = nullptr;
     gy_status st = GY_OK;
     const size_t rints = resort_scratch_ints(n) + 4 * (size_t)n;
     if (cudaMalloc(&mem, rints * sizeof(int) + 4096) != cudaSuccess) {
-        st = GY_ERR_NOMEM;
+        st = cuda_failed(GY_ERR_NOMEM);
     } else {
         int *d_key = mem, *d_prev = mem + n, *d_perm = mem + 2 * n, *d_sorted = mem + 3 * n;
         ResortScratch rs{};
@@ -1633,7 +1633,7 @@ gy_status gy_resort_keys(const int *keys, const int *prev_sorted, int64_t n, int
         resort_keys(d_key, d_prev, d_sorted, d_perm, n, bits, rs, s);
         cudaMemcpyAsync(perm_out, d_perm, n * sizeof(int), cudaMemcpyDeviceToHost, s);
         cudaMemcpyAsync(sorted_out, d_sorted, n * sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (cudaStreamSynchronize(s) != cudaSuccess) st = GY_ERR_CUDA;
+        if (cudaStreamSynchronize(s) != cudaSuccess) st = cuda_failed(GY_ERR_CUDA);
     }
     if (mem) cudaFree(mem);
     cudaStreamDestroy(s);

@@ -169,6 +169,14 @@ inline cudaError_t launch_step(void (*kernel)(P...), dim3 grid, dim3 block, cuda
     return cudaPeekAtLastError();
 }
 
+// The status of an entry point whose CUDA call failed: the runtime keeps such an error for whoever
+// asks it next (another handle's step or initialisation among them), so it is taken out with the answer.
+template <class Status> inline Status cuda_failed(Status st)
+{
+    cudaGetLastError();
+    return st;
+}
+
 // keeps the first failure of a sequence of launches (err may be null)
 inline void keep_first(cudaError_t *err, cudaError_t e)
 {

@@ -342,11 +342,11 @@ static int *g_static_addr[256] = {};
 static gy_status static_scratch(int **out)
 {
     int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 256) return GY_ERR_CUDA;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 256) return cuda_failed(GY_ERR_CUDA);
     std::lock_guard<std::mutex> lock(g_static_mu);
     if (!g_static_addr[dev]) {
         void *p = nullptr;
-        if (cudaGetSymbolAddress(&p, g_sort_static) != cudaSuccess || !p) return GY_ERR_CUDA;
+        if (cudaGetSymbolAddress(&p, g_sort_static) != cudaSuccess || !p) return cuda_failed(GY_ERR_CUDA);
         g_static_addr[dev] = static_cast<int *>(p);
     }
     *out = g_static_addr[dev];

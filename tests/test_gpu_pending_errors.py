@@ -1,0 +1,36 @@
+"""A call that fails on the host leaves no error behind in the CUDA runtime for the next call to
+answer for: handles initialise, step and answer as if nothing had happened."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from graphyt_gb300 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _no_such_device():
+    """A gy_create that fails on the host: there is no such device."""
+    from graphyt_gb300 import _lib
+    g = _lib.GridDesc()
+    g.L[:] = [1.0, 1.0, 1.0]
+    g.cellsize, g.psep = 0.125, 0.0625
+    h = C.c_void_p()
+    assert _lib.load().gy_create(C.byref(g), 9999, C.byref(h)) != 0
+
+
+def test_a_failed_call_leaves_no_error_behind(gpu_lib):
+    from graphyt_gb300 import _lib, graphyt
+    _no_such_device()
+    s = graphyt.from_scene(scenes.two_blocks())
+    s.iterate_GPU_steps(2)
+    s.close()
+    _no_such_device()
+    prm = torch.ones(int(gpu_lib.gy_mlp_param_count()), device="cuda")
+    X, Y = torch.zeros(5, 16, device="cuda"), torch.full((5, 7), np.nan, device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _lib.check(gpu_lib.gy_mlp_forward(p(prm), p(X), 5, p(Y), None, stream))
+    assert torch.isfinite(Y).all()
