@@ -1265,10 +1265,10 @@ static ExportArgs export_args(const gy_solver *h)
 static_assert(PF_PID < PF_EQPS && (PF_PID + 1) * 4 >= 6 * 8, "the getters' rows must fit the fields every step writes");
 static void *export_rows(gy_solver *h) { return h->slab[h->cur ^ 1]; }
 
-static gy_status copy_rows(gy_solver *h, void *out, size_t bytes)
+static gy_status copy_rows(gy_solver *h, cudaError_t launched, void *out, size_t bytes)
 {
-    const cudaError_t le = cudaGetLastError();
-    if (le != cudaSuccess) return fail(h, GY_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(le));
+    if (launched != cudaSuccess)
+        return fail(h, GY_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(launched));
     if (bytes) CK(h, cudaMemcpyAsync(out, export_rows(h), bytes, cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
     return GY_OK;
@@ -1301,6 +1301,7 @@ gy_status gy_get_particles(gy_solver *h, int field, double *out, int64_t count)
         return GY_OK;
     }
     cudaSetDevice(h->device);
+    cudaError_t launched;
     if (field == GY_P_TEMP || field == GY_P_TEMPGRAD) {
         // kept by insertion index; without a device copy every temperature is the host value
         // and every gradient zero
@@ -1308,11 +1309,11 @@ gy_status gy_get_particles(gy_solver *h, int field, double *out, int64_t count)
             for (long long i = 0; i < n * w; i++) out[i] = field == GY_P_TEMP ? h->temp[i] : 0.0;
             return GY_OK;
         }
-        launch_export_therm(h->d_therm, n, field, static_cast<double *>(export_rows(h)), h->stream);
+        launched = launch_export_therm(h->d_therm, n, field, static_cast<double *>(export_rows(h)), h->stream);
     } else {
-        launch_export(pview(h, h->cur), n, field, export_args(h), static_cast<double *>(export_rows(h)), h->stream);
+        launched = launch_export(pview(h, h->cur), n, field, export_args(h), static_cast<double *>(export_rows(h)), h->stream);
     }
-    return copy_rows(h, out, (size_t)count * sizeof(double));
+    return copy_rows(h, launched, out, (size_t)count * sizeof(double));
 }
 
 gy_status gy_get_particles_int(gy_solver *h, int field, int *out, int64_t count)
@@ -1335,8 +1336,9 @@ gy_status gy_get_particles_int(gy_solver *h, int field, int *out, int64_t count)
     }
     if (field < GY_PI_CELLID || field > GY_PI_DEVICE_SLOT) return GY_ERR_ARG;
     cudaSetDevice(h->device);
-    launch_export_int(pview(h, h->cur), n, field, export_args(h), static_cast<int *>(export_rows(h)), h->stream);
-    return copy_rows(h, out, (size_t)count * sizeof(int));
+    const cudaError_t launched =
+        launch_export_int(pview(h, h->cur), n, field, export_args(h), static_cast<int *>(export_rows(h)), h->stream);
+    return copy_rows(h, launched, out, (size_t)count * sizeof(int));
 }
 
 gy_status gy_get_nodes(gy_solver *h, int field, double *out, int64_t count)

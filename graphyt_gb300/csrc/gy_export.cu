@@ -112,22 +112,22 @@ __global__ void __launch_bounds__(256) k_export_therm(const float4 *therm, long 
 
 static unsigned export_grid(long long n) { return (unsigned)std::max(1ll, std::min((n + 255) / 256, 65536ll)); }
 
-void launch_export(const PView &p, long long n, int field, const ExportArgs &a, double *out, cudaStream_t s)
+cudaError_t launch_export(const PView &p, long long n, int field, const ExportArgs &a, double *out, cudaStream_t s)
 {
-    k_export<<<export_grid(n), 256, 0, s>>>(p, n, field, a, out);
     note_launch(1);
+    return launch_checked(k_export, export_grid(n), 256, s, p, n, field, a, out);
 }
 
-void launch_export_int(const PView &p, long long n, int field, const ExportArgs &a, int *out, cudaStream_t s)
+cudaError_t launch_export_int(const PView &p, long long n, int field, const ExportArgs &a, int *out, cudaStream_t s)
 {
-    k_export_int<<<export_grid(n), 256, 0, s>>>(p, n, field, a, out);
     note_launch(1);
+    return launch_checked(k_export_int, export_grid(n), 256, s, p, n, field, a, out);
 }
 
-void launch_export_therm(const float4 *therm, long long n, int field, double *out, cudaStream_t s)
+cudaError_t launch_export_therm(const float4 *therm, long long n, int field, double *out, cudaStream_t s)
 {
-    k_export_therm<<<export_grid(n), 256, 0, s>>>(therm, n, field, out);
     note_launch(1);
+    return launch_checked(k_export_therm, export_grid(n), 256, s, therm, n, field, out);
 }
 
 }  // namespace gy

@@ -169,6 +169,17 @@ inline cudaError_t launch_step(void (*kernel)(P...), dim3 grid, dim3 block, cuda
     return cudaPeekAtLastError();
 }
 
+// a plain launch that answers for itself: what another call left pending in the runtime is not its
+template <typename... P, typename... A>
+inline cudaError_t launch_checked(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A &&... args)
+{
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.stream = s;
+    return cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+}
+
 // The status of an entry point whose CUDA call failed: the runtime keeps such an error for whoever
 // asks it next (another handle's step or initialisation among them), so it is taken out with the answer.
 template <class Status> inline Status cuda_failed(Status st)
@@ -274,9 +285,9 @@ struct ExportArgs {
     bool has_dp, normals;
     int slot_obj[MAX_BODIES];
 };
-void launch_export(const PView &p, long long n, int field, const ExportArgs &a, double *out, cudaStream_t s);
-void launch_export_int(const PView &p, long long n, int field, const ExportArgs &a, int *out, cudaStream_t s);
-void launch_export_therm(const float4 *therm, long long n, int field, double *out, cudaStream_t s);
+cudaError_t launch_export(const PView &p, long long n, int field, const ExportArgs &a, double *out, cudaStream_t s);
+cudaError_t launch_export_int(const PView &p, long long n, int field, const ExportArgs &a, int *out, cudaStream_t s);
+cudaError_t launch_export_therm(const float4 *therm, long long n, int field, double *out, cudaStream_t s);
 // err (may be null) receives the first launch failure of the sort's kernels
 const int *sort_pairs(const int *keys_in, int *perm_out, long long n, int key_bits, SortScratch &ws, cudaStream_t s,
                       cudaError_t *err = nullptr);

@@ -34,3 +34,15 @@ def test_a_failed_call_leaves_no_error_behind(gpu_lib):
     stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
     _lib.check(gpu_lib.gy_mlp_forward(p(prm), p(X), 5, p(Y), None, stream))
     assert torch.isfinite(Y).all()
+
+
+def test_getters_are_not_refused_for_another_handles_error(gpu_lib):
+    from graphyt_gb300 import graphyt
+    s = graphyt.from_scene(scenes.two_blocks())
+    s.iterate_GPU_steps(2)
+    want = s._get_particles("pos"), s._get_particles_int("material")
+    _no_such_device()
+    got = s._get_particles("pos"), s._get_particles_int("material")
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
+    s.close()
