@@ -1115,6 +1115,35 @@ static void issue_step(gy_solver *h, const StepVariant &v, cudaEvent_t *tev)
     if (tev) cudaEventRecord(tev[4], s);
 }
 
+// The device's ring counter and the host's back at the first slot; the stream is idle.
+static gy_status reset_ring(gy_solver *h)
+{
+    h->ring_pos = 0;
+    std::fill(h->ring_busy, h->ring_busy + gy_solver::kRing / gy_solver::kGroup, false);
+    CK(h, cudaMemsetAsync(h->d_taken, 0, sizeof(int), h->stream));
+    return GY_OK;
+}
+
+// A launch of the step failed, and the kernels before it may have run: what they leave for the next
+// ones (the ring counter, the counts and movers of the sorts, segment counts, node sums) is reset,
+// so that the step can be tried again from the particles as they were.
+static gy_status drop_step(gy_solver *h, cudaError_t why)
+{
+    const std::string msg = std::string("kernel launch: ") + cudaGetErrorString(why);
+    const size_t row = (size_t)h->nn * sizeof(float4);
+    cudaStreamSynchronize(h->stream);
+    reset_ring(h);
+    h->since_sort = 1 << 30;
+    h->resort_valid = h->blocks_valid = false;
+    cudaMemsetAsync(h->d_nseg, 0, 4 * sizeof(int), h->stream);
+    float4 *sums[] = {h->nb.acc0, h->nb.acc1, h->nb.bacc0[0], h->nb.bacc1[0], h->nb.bnrm[0], h->nb.bacc0[1],
+                      h->nb.bacc1[1], h->nb.bnrm[1]};
+    for (float4 *p : sums)
+        if (p) cudaMemsetAsync(p, 0, row, h->stream);
+    if (h->d_tnode) cudaMemsetAsync(h->d_tnode, 0, (size_t)h->nn * sizeof(float2), h->stream);
+    return fail(h, GY_ERR_CUDA, msg);
+}
+
 static gy_status enqueue_step(gy_solver *h, double t, int step)
 {
     cudaStream_t s = h->stream;
@@ -1129,7 +1158,6 @@ static gy_status enqueue_step(gy_solver *h, double t, int step)
             h->tev.push_back(e);
         }
         tev = &h->tev[(size_t)h->tev_used * 5];
-        h->tev_used++;
     }
     // host decisions for this step
     StepVariant v{h->cur, h->sk, 0, 0, 0, h->fb};
@@ -1158,31 +1186,33 @@ static gy_status enqueue_step(gy_solver *h, double t, int step)
             StepGraph ng{};
             ng.v = v;
             const long long l0 = launch_count();
+            cudaGetLastError();  // an error that another call left is not this step's
             CK(h, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
             issue_step(h, v, nullptr);
+            cudaError_t ei = cudaGetLastError();
             cudaGraph_t graph = nullptr;
-            CK(h, cudaStreamEndCapture(s, &graph));
+            const cudaError_t ec = cudaStreamEndCapture(s, &graph);
+            if (ei == cudaSuccess) ei = ec;
             ng.launches = launch_count() - l0;
-            const cudaError_t ei = cudaGraphInstantiate(&ng.exec, graph, 0);
-            cudaGraphDestroy(graph);
-            if (ei != cudaSuccess) return fail(h, GY_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ei));
-            note_launch(-(int)ng.launches);  // counted again per replay below
+            note_launch(-(int)ng.launches);  // counted per replay below
+            if (ei == cudaSuccess) ei = cudaGraphInstantiate(&ng.exec, graph, 0);
+            if (graph) cudaGraphDestroy(graph);
+            if (ei != cudaSuccess)  // nothing has run
+                return fail(h, GY_ERR_CUDA, std::string("step graph: ") + cudaGetErrorString(ei));
             h->graphs.push_back(ng);
             gr = &h->graphs.back();
         }
         CK(h, cudaGraphLaunch(gr->exec, s));
         note_launch((int)gr->launches);
     } else {
+        cudaGetLastError();
         issue_step(h, v, tev);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return drop_step(h, e);
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(h, GY_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
-    // host bookkeeping
+    // the step is submitted: the host follows, whatever the calls after it return
+    if (timing) h->tev_used++;
     h->ring_pos++;
-    if (slot % gy_solver::kGroup == gy_solver::kGroup - 1) {
-        CK(h, cudaEventRecord(h->ring_ev[group], s));
-        h->ring_busy[group] = true;
-    }
     if (v.sort) {
         h->sk = v.sk;
         h->since_sort = 0;
@@ -1197,6 +1227,10 @@ static gy_status enqueue_step(gy_solver *h, double t, int step)
     h->t_prev = t;
     h->steps++;
     h->stats_fresh = true;
+    if (slot % gy_solver::kGroup == gy_solver::kGroup - 1) {
+        h->ring_busy[group] = cudaEventRecord(h->ring_ev[group], s) == cudaSuccess;
+        if (!h->ring_busy[group]) CK(h, cudaStreamSynchronize(s));
+    }
     return GY_OK;
 }
 
@@ -1556,7 +1590,8 @@ gy_status gy_state_load(gy_solver *h, const void *buf, int64_t bytes)
     h->since_sort = 1 << 30;
     h->resort_valid = false;
     h->blocks_valid = false;
-    return sum_state(h);
+    gy_status st = reset_ring(h);
+    return st ? st : sum_state(h);
 }
 
 gy_status gy_sort_keys(const int *keys, int64_t n, int *perm_out, int device)
