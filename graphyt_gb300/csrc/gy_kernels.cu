@@ -849,7 +849,9 @@ constexpr int PW_RUNS = 32;                          // most cells of a chunk (2
 __device__ __forceinline__ void gimp_axis_flat(float u, const GridGeom &g, float S[3], float G[3])
 {
     const float d = u - (1.0f - g.lp);
-    const float q = fmaxf(d, 0.0f), a = 2.0f * g.lp - q;
+    float q;  // max(d, 0), NaN where the offset is (fmaxf would make it 0)
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(q) : "f"(d));
+    const float a = 2.0f * g.lp - q;
     S[0] = fmaf(a * g.inv_4l, a, fmaxf(-d, 0.0f));
     S[2] = q * g.inv_4l * q;
     S[1] = 1.0f - S[0] - S[2];
