@@ -85,3 +85,36 @@ def test_a_pile_crossing_a_block_boundary_takes_no_longer_than_its_size(gpu_lib)
         s = graphyt.from_scene(sc)
     s.close()
     assert min(worst) < 0.05
+
+
+@pytest.mark.parametrize("L", [(5.25, 5.25, 4.75), (10.25, 10.25, 10.25)])
+def test_the_cluster_scan_gives_the_stable_sort(gpu_lib, tmp_path, L):
+    """Grids of 8,379 and 68,921 cell blocks, just above and well above what one CTA scans, no multiple
+    of four or eight: particles all over them, so that every CTA of the cluster has blocks with movers
+    in and out, land slot for slot where a sort from scratch puts them."""
+    from graphyt_gb300 import graphyt, scenes
+    rng = np.random.default_rng(11)
+    n = 60000
+    pos = 0.2 + rng.random((n, 3)) * (np.array(L) - 0.5)
+    vel = rng.uniform(-1.5, 1.5, (n, 3))
+    zero = np.zeros(n, np.int32)
+    base = scenes.tiny_block(model=1, n_side=4, cellsize=H)
+    base.materials[0].update(bulkMod=1.0, shearMod=0.5)
+    sc = scenes._finish(scenes.Scene("spread", list(L), H, H / 2, pos, zero, zero.copy(), base.materials, CFL=0.3, vel=vel),
+                        None)
+    sc.dt = 0.2 * H
+    a = graphyt.from_scene(sc)
+    b = graphyt.from_scene(sc, options=dict(full_sort=1))
+    a.iterate_GPU_steps(2)
+    for k in range(2, 8):
+        a.save(str(tmp_path / "s"))
+        b.load(str(tmp_path / "s"))
+        before = a._get_particles_int("device_slot")
+        for s in (a, b):
+            s.iterate_GPU(k * sc.dt, k)
+        slots = a._get_particles_int("device_slot")
+        assert np.array_equal(np.sort(slots), np.arange(n)), k
+        assert np.array_equal(slots, b._get_particles_int("device_slot")), k
+        assert np.mean(slots != before) > 0.5, k
+    a.close()
+    b.close()
