@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(PP_THREADS, THERMAL ? GY_PP_MINB_TH : GY_PP_MI
     for (int sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
         prefetch_next_segment(P, perm, sg, nseg, sgi + gridDim.x, PF_OX, PF_S5 + 1);
         prefetch_next_segment(P, perm, sg, nseg, sgi + gridDim.x, PF_RHO, PF_MASS + 1);
-        const long long start = sg.start[sgi], end = sg.len ? start + sg.len[sgi] : n;
+        const long long start = sg.start[sgi];
         const int blk = seg_block(skey, start);
         int bx, by, bz;
         decode_block(blk, g, bx, by, bz);
@@ -591,18 +591,13 @@ __global__ void __launch_bounds__(PP_THREADS, THERMAL ? GY_PP_MINB_TH : GY_PP_MI
             int cnt, ka = -1, kb = -1, kp = -1;
             long long ja = 0, jb = 0;
             if (sorted) {
-                ka = ia < end ? skey[ia] : -1;
-                kb = ib < end ? skey[ib] : -1;
-                kp = (ia < end && tid > 0) ? skey[ia - 1] : -1;
-                ja = ia < end ? perm[ia] : 0;
-                jb = ib < end ? perm[ib] : 0;
-                if (sg.len) {
-                    cnt = (int)min((long long)PP_CH, end - base);
-                    __syncthreads();
-                } else {
-                    cnt = __syncthreads_count(ia < end && (ka >> CB_SHIFT) == blk);
-                    cnt += __syncthreads_count(ib < end && (kb >> CB_SHIFT) == blk);
-                }
+                ka = ia < n ? skey[ia] : -1;
+                kb = ib < n ? skey[ib] : -1;
+                kp = (ia < n && tid > 0) ? skey[ia - 1] : -1;
+                ja = ia < n ? perm[ia] : 0;
+                jb = ib < n ? perm[ib] : 0;
+                cnt = __syncthreads_count(ia < n && (ka >> CB_SHIFT) == blk);
+                cnt += __syncthreads_count(ib < n && (kb >> CB_SHIFT) == blk);
             } else {
                 cnt = (int)min((long long)PP_CH, segment_chunk_end2(skey, n, blk, base, &s_end) - base);
                 if (2 * tid < cnt) {
@@ -1674,7 +1669,6 @@ __device__ __forceinline__ void contact_normal(const float rv[3], const float n[
 }
 
 // One node of an active node block; returns whether the node carries mass.
-template <bool MULTI>
 __device__ __forceinline__ bool solve_node(const NodeBufs &nb, const StepArgs &a, int keep, long long blk, int lnode)
 {
     const GridGeom &g = a.g;
@@ -1688,127 +1682,109 @@ __device__ __forceinline__ bool solve_node(const NodeBufs &nb, const StepArgs &a
         if (i < g.nx && j < g.ny && k < g.nz) {
             const int nd = node_index(i, j, k, g);
             const float4 A0 = nb.acc0[nd];
-            float4 A1 = nb.acc1[nd];
+            const float4 A1 = nb.acc1[nd];
             const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
             // every load of the node is issued before the first store (the accumulators are
             // cleared after they were read)
             float4 B0[2], B1[2], BN[2];
-            int2 body = make_int2(-1, -1);
-            unsigned char hr = 0;
             // a node block whose nodes all hold one body has nothing in slot 1, and its nodes
             // need no normal unless normals are tracked
-            bool two = false;
-            if (MULTI) {
-                two = nb.nblk_two[blk] != 0;
-                B0[0] = nb.bacc0[0][nd];
-                B1[0] = nb.bacc1[0][nd];
-                body = nb.body[nd];
-                hr = nb.has_rigid[nd];
-                BN[0] = (two || nb.nrm_out[0]) ? nb.bnrm[0][nd] : z4;
-                B0[1] = B1[1] = BN[1] = z4;
-                if (two) {
-                    B0[1] = nb.bacc0[1][nd];
-                    B1[1] = nb.bacc1[1][nd];
-                    BN[1] = nb.bnrm[1][nd];
-                }
+            const bool two = nb.nblk_two[blk] != 0;
+            B0[0] = nb.bacc0[0][nd];
+            B1[0] = nb.bacc1[0][nd];
+            const int2 body = nb.body[nd];
+            const unsigned char hr = nb.has_rigid[nd];
+            BN[0] = (two || nb.nrm_out[0]) ? nb.bnrm[0][nd] : z4;
+            B0[1] = B1[1] = BN[1] = z4;
+            if (two) {
+                B0[1] = nb.bacc0[1][nd];
+                B1[1] = nb.bacc1[1][nd];
+                BN[1] = nb.bnrm[1][nd];
             }
             const int bt = nb.bc_type ? nb.bc_type[nd] : 0;
             nb.acc0[nd] = z4;
             nb.acc1[nd] = z4;
             const float m = A0.x;
-            if (!MULTI) {
-                // single body: gravity enters here as m_node * g (Extrapolation.cpp:226-228)
-                A1.x += m * a.sc->gravity[0];
-                A1.y += m * a.sc->gravity[1];
-                A1.z += m * a.sc->gravity[2];
-            }
             const float dtn = a.sc->dt_node, dt = a.sc->dt;
             float vc[3] = {0.f, 0.f, 0.f};
             float v1[3] = {0.f, 0.f, 0.f}, a1[3] = {0.f, 0.f, 0.f};
             float v2[3] = {0.f, 0.f, 0.f}, a2[3] = {0.f, 0.f, 0.f};
             float n1[3] = {0.f, 0.f, 0.f};
             active = (m != 0.0f);
-            if (!MULTI) {
-                if (active) {
-                    vc[0] = A0.y / m; vc[1] = A0.z / m; vc[2] = A0.w / m;
-                    body_update(m, A0, A1, dtn, v1, a1);
-                }
-            } else {
-                nb.bacc0[0][nd] = z4;
-                nb.bacc1[0][nd] = z4;
-                nb.bnrm[0][nd] = z4;
-                if (two) {
-                    nb.bacc0[1][nd] = z4;
-                    nb.bacc1[1][nd] = z4;
-                    nb.bnrm[1][nd] = z4;
-                }
-                if (active) {
-                    vc[0] = A0.y / m; vc[1] = A0.z / m; vc[2] = A0.w / m;
-                    const float mag1 = sqrtf(BN[0].x * BN[0].x + BN[0].y * BN[0].y + BN[0].z * BN[0].z);
-                    if (mag1 > 1e-8f) { n1[0] = BN[0].x / mag1; n1[1] = BN[0].y / mag1; n1[2] = BN[0].z / mag1; }
-                    const float n2[3] = {-n1[0], -n1[1], -n1[2]};  // Grid.cpp:45-47
-                    const float m1 = B0[0].x, m2 = B0[1].x;
-                    if (body.y != -1) {
-                        float ap1 = 0.f, ap2 = 0.f, rv1[3] = {0.f, 0.f, 0.f}, rv2[3] = {0.f, 0.f, 0.f};
-                        if (m1 != 0.0f) {
-                            rv1[0] = B0[0].y / m1 - vc[0]; rv1[1] = B0[0].z / m1 - vc[1]; rv1[2] = B0[0].w / m1 - vc[2];
-                            ap1 = rv1[0] * n1[0] + rv1[1] * n1[1] + rv1[2] * n1[2];
-                        }
-                        if (m2 != 0.0f) {
-                            rv2[0] = B0[1].y / m2 - vc[0]; rv2[1] = B0[1].z / m2 - vc[1]; rv2[2] = B0[1].w / m2 - vc[2];
-                            ap2 = rv2[0] * n2[0] + rv2[1] * n2[1] + rv2[2] * n2[2];
-                        }
-                        if (ap1 > 0.01f || ap2 > 0.01f) {
-                            if (hr & 1) {
-                                // body 1 rigid: body 2 takes body 1's velocity (Grid.cpp:78-91)
-                                if (m1 != 0.0f) {
-                                    v1[0] = B0[0].y / m1; v1[1] = B0[0].z / m1; v1[2] = B0[0].w / m1;
-                                    if (m2 != 0.0f) {
-                                        v2[0] = B0[1].y / m2 - (B0[1].y - m2 * v1[0]) / m2;
-                                        v2[1] = B0[1].z / m2 - (B0[1].z - m2 * v1[1]) / m2;
-                                        v2[2] = B0[1].w / m2 - (B0[1].w - m2 * v1[2]) / m2;
-                                    }
-                                }
-                            } else if (hr & 2) {
+            nb.bacc0[0][nd] = z4;
+            nb.bacc1[0][nd] = z4;
+            nb.bnrm[0][nd] = z4;
+            if (two) {
+                nb.bacc0[1][nd] = z4;
+                nb.bacc1[1][nd] = z4;
+                nb.bnrm[1][nd] = z4;
+            }
+            if (active) {
+                vc[0] = A0.y / m; vc[1] = A0.z / m; vc[2] = A0.w / m;
+                const float mag1 = sqrtf(BN[0].x * BN[0].x + BN[0].y * BN[0].y + BN[0].z * BN[0].z);
+                if (mag1 > 1e-8f) { n1[0] = BN[0].x / mag1; n1[1] = BN[0].y / mag1; n1[2] = BN[0].z / mag1; }
+                const float n2[3] = {-n1[0], -n1[1], -n1[2]};  // Grid.cpp:45-47
+                const float m1 = B0[0].x, m2 = B0[1].x;
+                if (body.y != -1) {
+                    float ap1 = 0.f, ap2 = 0.f, rv1[3] = {0.f, 0.f, 0.f}, rv2[3] = {0.f, 0.f, 0.f};
+                    if (m1 != 0.0f) {
+                        rv1[0] = B0[0].y / m1 - vc[0]; rv1[1] = B0[0].z / m1 - vc[1]; rv1[2] = B0[0].w / m1 - vc[2];
+                        ap1 = rv1[0] * n1[0] + rv1[1] * n1[1] + rv1[2] * n1[2];
+                    }
+                    if (m2 != 0.0f) {
+                        rv2[0] = B0[1].y / m2 - vc[0]; rv2[1] = B0[1].z / m2 - vc[1]; rv2[2] = B0[1].w / m2 - vc[2];
+                        ap2 = rv2[0] * n2[0] + rv2[1] * n2[1] + rv2[2] * n2[2];
+                    }
+                    if (ap1 > 0.01f || ap2 > 0.01f) {
+                        if (hr & 1) {
+                            // body 1 rigid: body 2 takes body 1's velocity (Grid.cpp:78-91)
+                            if (m1 != 0.0f) {
+                                v1[0] = B0[0].y / m1; v1[1] = B0[0].z / m1; v1[2] = B0[0].w / m1;
                                 if (m2 != 0.0f) {
-                                    v2[0] = B0[1].y / m2; v2[1] = B0[1].z / m2; v2[2] = B0[1].w / m2;
-                                    if (m1 != 0.0f) {
-                                        v1[0] = B0[0].y / m1 - (B0[0].y - m1 * v2[0]) / m1;
-                                        v1[1] = B0[0].z / m1 - (B0[0].z - m1 * v2[1]) / m1;
-                                        v1[2] = B0[0].w / m1 - (B0[0].w - m1 * v2[2]) / m1;
-                                    }
+                                    v2[0] = B0[1].y / m2 - (B0[1].y - m2 * v1[0]) / m2;
+                                    v2[1] = B0[1].z / m2 - (B0[1].z - m2 * v1[1]) / m2;
+                                    v2[2] = B0[1].w / m2 - (B0[1].w - m2 * v1[2]) / m2;
                                 }
-                            } else {
+                            }
+                        } else if (hr & 2) {
+                            if (m2 != 0.0f) {
+                                v2[0] = B0[1].y / m2; v2[1] = B0[1].z / m2; v2[2] = B0[1].w / m2;
                                 if (m1 != 0.0f) {
-                                    float cn[3];
-                                    contact_normal(rv1, n1, a.sc->mu, cn);
-                                    v1[0] = B0[0].y / m1 - ap1 * cn[0];
-                                    v1[1] = B0[0].z / m1 - ap1 * cn[1];
-                                    v1[2] = B0[0].w / m1 - ap1 * cn[2];
-                                    a1[0] = B1[0].x / m1 - (ap1 * cn[0]) / dt;
-                                    a1[1] = B1[0].y / m1 - (ap1 * cn[1]) / dt;
-                                    a1[2] = B1[0].z / m1 - (ap1 * cn[2]) / dt;
-                                    for (int c = 0; c < 3; c++) v1[c] += a1[c] * dtn;
-                                }
-                                if (m2 != 0.0f) {
-                                    float cn[3];
-                                    contact_normal(rv2, n2, a.sc->mu, cn);
-                                    v2[0] = B0[1].y / m2 - ap2 * cn[0];
-                                    v2[1] = B0[1].z / m2 - ap2 * cn[1];
-                                    v2[2] = B0[1].w / m2 - ap2 * cn[2];
-                                    a2[0] = B1[1].x / m2 - (ap2 * cn[0]) / dt;
-                                    a2[1] = B1[1].y / m2 - (ap2 * cn[1]) / dt;
-                                    a2[2] = B1[1].z / m2 - (ap2 * cn[2]) / dt;
-                                    for (int c = 0; c < 3; c++) v2[c] += a2[c] * dtn;
+                                    v1[0] = B0[0].y / m1 - (B0[0].y - m1 * v2[0]) / m1;
+                                    v1[1] = B0[0].z / m1 - (B0[0].z - m1 * v2[1]) / m1;
+                                    v1[2] = B0[0].w / m1 - (B0[0].w - m1 * v2[2]) / m1;
                                 }
                             }
                         } else {
-                            if (m1 != 0.0f) body_update(m1, B0[0], B1[0], dtn, v1, a1);
-                            if (m2 != 0.0f) body_update(m2, B0[1], B1[1], dtn, v2, a2);
+                            if (m1 != 0.0f) {
+                                float cn[3];
+                                contact_normal(rv1, n1, a.sc->mu, cn);
+                                v1[0] = B0[0].y / m1 - ap1 * cn[0];
+                                v1[1] = B0[0].z / m1 - ap1 * cn[1];
+                                v1[2] = B0[0].w / m1 - ap1 * cn[2];
+                                a1[0] = B1[0].x / m1 - (ap1 * cn[0]) / dt;
+                                a1[1] = B1[0].y / m1 - (ap1 * cn[1]) / dt;
+                                a1[2] = B1[0].z / m1 - (ap1 * cn[2]) / dt;
+                                for (int c = 0; c < 3; c++) v1[c] += a1[c] * dtn;
+                            }
+                            if (m2 != 0.0f) {
+                                float cn[3];
+                                contact_normal(rv2, n2, a.sc->mu, cn);
+                                v2[0] = B0[1].y / m2 - ap2 * cn[0];
+                                v2[1] = B0[1].z / m2 - ap2 * cn[1];
+                                v2[2] = B0[1].w / m2 - ap2 * cn[2];
+                                a2[0] = B1[1].x / m2 - (ap2 * cn[0]) / dt;
+                                a2[1] = B1[1].y / m2 - (ap2 * cn[1]) / dt;
+                                a2[2] = B1[1].z / m2 - (ap2 * cn[2]) / dt;
+                                for (int c = 0; c < 3; c++) v2[c] += a2[c] * dtn;
+                            }
                         }
                     } else {
                         if (m1 != 0.0f) body_update(m1, B0[0], B1[0], dtn, v1, a1);
+                        if (m2 != 0.0f) body_update(m2, B0[1], B1[1], dtn, v2, a2);
                     }
+                } else {
+                    if (m1 != 0.0f) body_update(m1, B0[0], B1[0], dtn, v1, a1);
                 }
             }
             // grid BC, phase 2 (phase 1 is overwritten by the solve for every node the
@@ -1827,17 +1803,15 @@ __device__ __forceinline__ bool solve_node(const NodeBufs &nb, const StepArgs &a
             }
             nb.gv[nd] = make_float4(m, v1[0], v1[1], v1[2]);
             nb.ga[nd] = make_float4(a1[0], a1[1], a1[2], 0.f);
-            if (MULTI && two) {
+            if (two) {
                 // slot 0's solved fields are gv / ga; slot 1 is read only where a node holds two
                 // bodies
                 nb.bgv[1][nd] = make_float4(m, v2[0], v2[1], v2[2]);
                 nb.bga[1][nd] = make_float4(a2[0], a2[1], a2[2], 0.f);
             }
-            if (MULTI) {
-                if (nb.nrm_out[0]) {
-                    nb.nrm_out[0][nd] = make_float4(n1[0], n1[1], n1[2], 0.f);
-                    nb.nrm_out[1][nd] = make_float4(-n1[0], -n1[1], -n1[2], 0.f);
-                }
+            if (nb.nrm_out[0]) {
+                nb.nrm_out[0][nd] = make_float4(n1[0], n1[1], n1[2], 0.f);
+                nb.nrm_out[1][nd] = make_float4(-n1[0], -n1[1], -n1[2], 0.f);
             }
             if (keep) {
                 nb.out_com[nd] = make_float4(vc[0], vc[1], vc[2], 0.f);
@@ -1943,7 +1917,6 @@ __global__ void __launch_bounds__(256) k_solve_single(NodeBufs nb, StepArgs a, i
 #ifndef GY_SOLVE_MINB
 #define GY_SOLVE_MINB 5  // resident 256-thread CTAs per SM the multi-body solve is register-capped to (48)
 #endif
-template <bool MULTI>
 __global__ void __launch_bounds__(256, GY_SOLVE_MINB) k_solve_multi(NodeBufs nb, StepArgs a, int keep, int want_list)
 {
     const int lane = threadIdx.x & 31;
@@ -1961,7 +1934,7 @@ __global__ void __launch_bounds__(256, GY_SOLVE_MINB) k_solve_multi(NodeBufs nb,
         for (; active; active &= active - 1u) {
             const int blk = w0 + (__ffs(active) - 1) * step;
             if (want_list && half == 0 && lane == 0) nb.active_list[atomicAdd(nb.active_n, 1)] = blk;
-            count += solve_node<MULTI>(nb, a, keep, blk, lane + 32 * half) ? 1 : 0;
+            count += solve_node(nb, a, keep, blk, lane + 32 * half) ? 1 : 0;
         }
     }
     if (nb.active_count) {
@@ -1981,7 +1954,7 @@ void launch_solve(const NodeBufs &nb, const StepArgs &a, bool keep_node_fields, 
     const int keep = keep_node_fields ? 1 : 0, list = want_list ? 1 : 0;
     const long long warps = a.multi_body ? 2 * a.g.nnb : a.g.nnb;
     const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>((warps + 7) / 8, (long long)sms * 16));
-    if (a.multi_body) launch_step(k_solve_multi<true>, grid, 256, s, nb, a, keep, list);
+    if (a.multi_body) launch_step(k_solve_multi, grid, 256, s, nb, a, keep, list);
     else launch_step(k_solve_single, grid, 256, s, nb, a, keep, list);
     note_launch(1);
 }
