@@ -88,7 +88,7 @@ struct gy_solver {
     int sk = 0;
     bool resort_valid = false;              // slab order = order of the sort in skey_buf[sk], and every
                                             // G2P since has flagged the movers
-    BlockSort bs{};                         // block merge sort (bs.nblk 0: the grid has too many blocks for it)
+    BlockSort bs{};                         // block merge sort (bs.nblk 0: too many blocks, or no room for it)
     void *blocks_mem = nullptr;
     int fb = 0;                             // bs.first[fb] is the last sort's
     bool blocks_valid = false;              // slab order = that sort's, one G2P since, which kept the counts
@@ -875,14 +875,6 @@ gy_status gy_initialize(gy_solver *h, const gy_material *mats, int nmat, const g
     if ((st = dalloc(h, &h->d_seg, (h->multi ? 2 : 1) * h->cap))) return st;
     if ((st = dalloc(h, &h->d_seglen, h->cap))) return st;
     if ((st = dalloc(h, &h->d_nseg, 4))) return st;
-    if (const long long nblk = (long long)h->g.nbx * h->g.nby * h->g.nbz; nblk <= BLOCK_SORT_MAX) {
-        const size_t bytes = block_sort_ints(nblk, h->cap) * sizeof(int);
-        CK(h, cudaMalloc(&h->blocks_mem, bytes));
-        CK(h, cudaMemsetAsync(h->blocks_mem, 0, bytes, h->stream));
-        block_sort_bind(h->bs, (int *)h->blocks_mem, nblk, h->cap);
-        h->fb = 0;
-    }
-    h->blocks_valid = false;
     CK(h, cudaMemsetAsync(h->d_nseg, 0, 4 * sizeof(int), h->stream));
     {
         int dev = 0, sms = 1;
@@ -894,6 +886,20 @@ gy_status gy_initialize(gy_solver *h, const gy_material *mats, int nmat, const g
     if ((st = alloc_nodes(h))) return st;
     for (long long i = 0; i < n && !h->thermal; i++) h->thermal = h->temp[i] != 0.0;
     if (h->thermal && (st = enable_thermal(h))) return st;
+    // the block merge sort, after everything a step cannot do without: its 32 to 40 bytes per particle
+    // are room for speed, and a problem that fills the device sorts by the re-sort instead
+    h->blocks_valid = false;
+    h->fb = 0;
+    if (const long long nblk = (long long)h->g.nbx * h->g.nby * h->g.nbz; nblk <= BLOCK_SORT_MAX) {
+        const size_t bytes = block_sort_ints(nblk, h->cap) * sizeof(int);
+        if (cudaMalloc(&h->blocks_mem, bytes) == cudaSuccess) {
+            CK(h, cudaMemsetAsync(h->blocks_mem, 0, bytes, h->stream));
+            block_sort_bind(h->bs, (int *)h->blocks_mem, nblk, h->cap);
+        } else {
+            h->blocks_mem = nullptr;
+            cudaGetLastError();
+        }
+    }
     // the slab goes to the device in insertion order; put it in cell-key order now, so the
     // first step reads it coalesced and re-sorts only the particles that move
     h->resort_valid = false;
