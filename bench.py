@@ -555,7 +555,7 @@ def measure(args, rank, world, local, dist):
                        "model": {"dam_break": "newtonian", "brazilian_disc": "drucker_prager+grady_kipp, 3 bodies",
                                  "impact_batch": "drucker_prager+grady_kipp slab + elastic sphere per instance, "
                                                  "2 bodies"}[args.workload],
-                       "sort_every": args.sort_every, "p2g_lanes": args.p2g_lanes, "sort": "full" if args.full_sort else "incremental", "l2": "state larger than L2 (no flush needed)",
+                       "sort_every": args.sort_every, "p2g_lanes": args.p2g_lanes, "sort": "full" if args.full_sort else "block merge" if args.sort_every == 1 else "incremental", "l2": "state larger than L2 (no flush needed)",
                        "parallelism": ("instances sharded" if sharded else "replicas") if world > 1 else "single"},
             "window": {"first_timed_step": step_timed0, "of_run_steps": RUN_STEPS[args.workload],
                        "movers_per_step": movers},

@@ -156,6 +156,11 @@ static constexpr long long kMaxTimedSteps = 4096;
 // eight per cell fill 23,000 blocks).  Step with the block merge / the re-sort, on grids of 33,000,
 // 262,000, 512,000 and 1,000,000 blocks: 41 / 123, 63 / 131, 86 / 138 and 129 / 148 us with 8,000
 // particles, 53 / 117, 75 / 126, 96 / 131 and 139 / 144 us with 97,000.
+// Cells fuller than eight particles are no reason for the re-sort: a block of many rounds takes its
+// CTA longer (sort phase by the block merge / the re-sort, in cells of 27, 64, 216 and 512 particles:
+// 21 / 55, 33 / 57, 77 / 54 and 193 / 53 us), but only the block merge gives P2G segments of bounded
+// length, and a run of 512 particles in one cell takes the P2G of whole blocks 5.5 ms against 0.07
+// (step of 262,000 particles, 512 to a cell: 0.28 / 6.7 ms; 64 to a cell: 0.12 / 0.48).
 static constexpr long long BLOCK_SORT_MAX = 1 << 20;
 
 // Particles per segment of a sorted step.  A segment is one warp's work in P2G and one CTA's in
@@ -171,6 +176,10 @@ static constexpr long long BLOCK_SORT_MAX = 1 << 20;
 // 133.1); with fewer the longer pieces make the tail longer (184,000 particles 63.2 -> 65.7 us),
 // and with several bodies, whose pieces are one chunk of a CTA, they take another pass (24 impacts
 // of 1.1 million 316 -> 319).
+// The body-slot kernels take the same pieces where they take every segment (track_normals, or
+// p2g_lanes = 9 with bodies); P2G of pieces / of whole blocks with tracked normals: disks 17 / 17 us,
+// disc of 11,000 20 / 52, 165,000 37 / 58, 1.3 million 180 / 181; impacts of 184,000 41 / 56, 426,000
+// 74 / 88, 1.1 million 159 / 176.
 static Pieces segment_pieces(long long n, bool multi)
 {
     if (n >= 4000000) return {10, 0};  // 1024: a full block of eight particles per cell holds 512

@@ -822,9 +822,12 @@ __global__ void __launch_bounds__(PP_THREADS, THERMAL ? GY_PP_MINB_TH : GY_PP_MI
 // from partition of unity) and the z weight and gradient of each plane.  The f_z sums of two
 // rows are packed like the x and y components of one, so that a particle costs a lane about 140
 // instructions (190 with the weights formed by each lane from the offsets, and f_z unpacked).
-// Tile and staging take 15.8 KB, 14 warps per SM.
+// Tile and staging take 15.6 KB (18.8 KB with heat conduction), which leaves room for 13 (11) warps per
+// SM; the launch bound of 14 only caps the registers (bounds of 13 and 11 measured the same: 730,000
+// particles 28.24 against 28.19 ms a pass, with heat conduction 21.8 against 22.1, 2.4 million 70.9
+// against 70.2).
 //
-// What bounds it is the latency of loads and instructions at those 14 warps: 49 % of the issue
+// What bounds it is the latency of loads and instructions at those 13 warps: 49 % of the issue
 // slots, 37 warp instructions per particle (26 with whole blocks as segments), DRAM at 13-25 % of
 // its peak.  P2G with the shared tile / this kernel: 21 / 11 us at 8,000 particles, 88 / 61 at
 // 730,000, 223 / 156 at 2.4 million, 850 / 625 at 12 million in a developed flow; disc of 1.3

@@ -116,7 +116,7 @@ __device__ __forceinline__ void take_scalars(const ScalarRing &r)
 
 struct StepArgs {
     GridGeom g;
-    const StepScalars *sc;   // per-step scalars in device memory (one small copy per step)
+    const StepScalars *sc;   // the step's scalars in device memory, where its first kernel put them (ScalarRing)
     int multi_body;          // host-side launch choice, fixed per handle
     const DevMaterial *mats;
     const float4 *pbc_val;   // particle BC values by pid
@@ -200,8 +200,10 @@ long long launch_count();
 
 // launchers (gy_kernels.cu)
 // therm / tnode non-null: the single-body kernel also sums the heat conduction node fields
-// (multi-body problems run launch_thermal_p2g instead).  lanes: lanes per run of equal cell in
-// the single-body kernel without heat conduction, 3 (z-plane lanes) or 9 (x-column lanes).
+// (multi-body problems run launch_thermal_p2g instead).  lanes: 3 takes the warp kernel where the
+// segments have lengths (steps sorted by block) and the z-plane kernel, three lanes per run of equal
+// cell, elsewhere; 9 the x-column kernel, nine lanes per run (with several bodies the body-slot kernel
+// throughout).  defer / ndefer: list and count of the segments left to the body-slot kernel.
 void launch_p2g(const PView &p, const int *perm, const int *skey, long long n, const Segs &sg,
                 int persist_grid, const NodeBufs &nb, const StepArgs &a, cudaStream_t s,
                 const float4 *therm = nullptr, float2 *tnode = nullptr, int lanes = 3, int *defer = nullptr,

@@ -79,7 +79,7 @@ typedef struct gy_options {
                            cell block (or an incremental re-sort of the particles that
                            changed cell, with sort_every > 1); same permutation */
     int use_graph;      /* 1 (default): each step replays a captured CUDA graph of its kernels,
-                           the step's scalars reaching the device in one small copy; 0: the
+                           the step's scalars taken from pinned memory by its first one; 0: the
                            kernels are launched one by one */
     int track_normals;  /* 1: keep per-particle contact normals (getNormalsArr) */
     int check_finite;   /* 1: flag NaN/Inf in particle state every step */
